@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "dfloat.cuh"
+#include "seeded.cuh"
 
 namespace pcfd {
 
@@ -139,6 +140,137 @@ __device__ __forceinline__ int roe_core(const RoeSide<S>& L, const RoeSide<S>& R
   const S zero = Sc<S>::c(0.0), tiny = Sc<S>::c(1.0e-10);
   return ((rL < zero || EL < tiny || PL < tiny) ? 1 : 0) | ((rR < zero || ER < tiny || PR < tiny) ? 2 : 0) |
          ((P < tiny || rE < tiny) ? 4 : 0);
+}
+
+// The FP64 form of the flux for the residual.  The FP64 pipe bounds every
+// kernel that evaluates it (88 % busy in the edge pass), so it is written for
+// few FP64 instructions, EDGE_INST an edge where the generic form compiles to
+// 256: reciprocals and roots from FP32 seeds (seeded.cuh); one reciprocal per
+// side; the acoustic speeds of the two sides, which only the entropy fix of
+// the acoustic eigenvalues reads, formed only where an FP32 test cannot rule
+// that fix out; the largest-difference selections and the non-physical tests
+// on the integer pipes.  The mass flux is the momentum dotted with the normal
+// (one rounding of the stored values instead of the velocity's), and each
+// component adds the physical parts to the upwind part in one chain of fused
+// multiply-adds: against quad precision its error is 0.83 of the generic
+// form's on random face states (Mach 0.8, +-1 % and +-0.05 % jumps).
+// Edge pass of the 128x96x96 box: 3.765 ms before, 2.106 ms now.
+struct Roe64Side {
+  double r, ir, u, v, w, E, P, h, rt, th;
+};
+
+__device__ __forceinline__ Roe64Side roe64_side(const double* Q, const double nx, const double ny, const double nz,
+                                                const double gm1) {
+  Roe64Side o;
+  o.r = Q[0];
+  o.ir = recip(o.r);
+  o.u = Q[1] * o.ir;
+  o.v = Q[2] * o.ir;
+  o.w = Q[3] * o.ir;
+  o.E = Q[4];
+  o.P = gm1 * fma(-0.5, fma(o.u, Q[1], fma(o.v, Q[2], o.w * Q[3])), o.E);
+  o.h = (o.E + o.P) * o.ir;
+  o.rt = fma(Q[1], nx, fma(Q[2], ny, Q[3] * nz));
+  o.th = o.rt * o.ir;
+  return o;
+}
+
+// |eig| with the Harten-Hyman fix (entropy_fix), selections on integer keys
+__device__ __forceinline__ double entropy_fix64(double eig, double eigL, double eigR) {
+  const double dl = eig - eigL, dr = eigR - eig;
+  double eps = key_gt(dl, dr) ? dl : dr;
+  if (!key_gt(eps, 0.0)) eps = 0.0;
+  const double a = abs_bits(eig);
+  return key_gt(eps, a) ? 0.5 * fma(eig * eig, recip(eps), eps) : a;
+}
+
+// Roe's flux (roe_flux), the same returned mask
+__device__ __forceinline__ int roe_flux64(const double* QL, const double* QR, const double nx, const double ny,
+                                          const double nz, const double area, const double gamma, const double gm1,
+                                          const double igamma, double* flux) {
+  const Roe64Side L = roe64_side(QL, nx, ny, nz, gm1), R = roe64_side(QR, nx, ny, nz, gm1);
+  // Roe-averaged state
+  const double rho = root(L.r * R.r);
+  const double sigma = rho * recip(L.r + rho);
+  const double u = fma(sigma, R.u - L.u, L.u);
+  const double v = fma(sigma, R.v - L.v, L.v);
+  const double w = fma(sigma, R.w - L.w, L.w);
+  const double h = fma(sigma, R.h - L.h, L.h);
+  const double v2h = 0.5 * fma(u, u, fma(v, v, w * w));
+  const double c2 = gm1 * (h - v2h);
+  double ic;
+  const double c = sqrt_inv(c2, &ic);
+  const double thetaf = fma(u, nx, fma(v, ny, w * nz));
+
+  // entropy-fixed |eigenvalues|; the fix of an acoustic one applies when
+  // |eig| is below the larger of its differences from the two sides' values.
+  // In FP32, each difference is at most |dtheta| + |dc| over the pair; the
+  // margin covers the estimates' errors (2^-20 of the speeds summed).
+  const double l0 = entropy_fix64(thetaf, L.th, R.th);
+  const double ep = thetaf + c, em = thetaf - c;
+  double l3 = abs_bits(ep), l4 = abs_bits(em);
+  {
+    const float fg = est_f32(gamma);
+    const float thf = est_f32(thetaf), cf = est_f32(c), thl = est_f32(L.th), thr = est_f32(R.th);
+    const float cl = sqrt_f32(fg * est_f32(L.P) * est_f32(L.ir)), cr = sqrt_f32(fg * est_f32(R.P) * est_f32(R.ir));
+    const float jump = fmaxf(fabsf(thf - thl), fabsf(thr - thf)) + fmaxf(fabsf(cf - cl), fabsf(cr - cf)) +
+                       1.0e-5f * (fabsf(thl) + fabsf(thr) + fabsf(thf) + cl + cr + cf);
+    if (!(fabsf(thf + cf) > jump && fabsf(thf - cf) > jump)) {
+      const double cL = root(gamma * L.P * L.ir), cR = root(gamma * R.P * R.ir);
+      l3 = entropy_fix<double>(ep, L.th + cL, R.th + cR);
+      l4 = entropy_fix<double>(em, L.th - cL, R.th - cR);
+    }
+  }
+
+  // |A| dQ in projector form (see roe_core)
+  const double d0 = QR[0] - QL[0], d1 = QR[1] - QL[1], d2 = QR[2] - QL[2], d3 = QR[3] - QL[3], d4 = QR[4] - QL[4];
+  const double rdvn = fma(-thetaf, d0, fma(nx, d1, fma(ny, d2, nz * d3)));
+  const double dp = gm1 * fma(v2h, d0, fma(-u, d1, fma(-v, d2, fma(-w, d3, d4))));
+  const double hic2 = 0.5 * ic * ic;
+  const double ap3 = (l3 - l0) * (fma(c, rdvn, dp) * hic2);
+  const double ap4 = (l4 - l0) * (fma(-c, rdvn, dp) * hic2);
+  const double sp = ap3 + ap4, sm = c * (ap3 - ap4);
+  const double dr0 = fma(l0, d0, sp);
+  const double dr1 = fma(l0, d1, fma(u, sp, nx * sm));
+  const double dr2 = fma(l0, d2, fma(v, sp, ny * sm));
+  const double dr3 = fma(l0, d3, fma(w, sp, nz * sm));
+  const double dr4 = fma(l0, d4, fma(h, sp, thetaf * sm));
+
+  // 0.5 area (F_L + F_R - |A| dQ), F the physical flux (Flux, :686)
+  const double ha = 0.5 * area;
+  const double ps = L.P + R.P;
+  flux[0] = ha * ((L.rt + R.rt) - dr0);
+  flux[1] = ha * fma(ps, nx, fma(L.u, L.rt, fma(R.u, R.rt, -dr1)));
+  flux[2] = ha * fma(ps, ny, fma(L.v, L.rt, fma(R.v, R.rt, -dr2)));
+  flux[3] = ha * fma(ps, nz, fma(L.w, L.rt, fma(R.w, R.rt, -dr3)));
+  flux[4] = ha * (fma(L.h, L.rt, R.h * R.rt) - dr4);
+
+  // BadExtrapolation of the three states.  The pressure and energy of the
+  // Roe state are rho c2 / gamma and at least 1 / (gamma - 1) of it; all
+  // clearly above the threshold, on the high words and for the product in
+  // FP32, means no flag.
+  const int lim = 0x3ddb7cdf;  // high word of 1e-10
+  const bool clear = __double2hiint(L.r) >= 0 && __double2hiint(R.r) >= 0 && __double2hiint(L.E) > lim &&
+                     __double2hiint(R.E) > lim && __double2hiint(L.P) > lim && __double2hiint(R.P) > lim &&
+                     est_f32(rho) * est_f32(c2) > 1.0e-9f * est_f32(gamma) * (1.0f + est_f32(gm1));
+  if (clear) return 0;
+  const double zero = 0.0, tiny = 1.0e-10;
+  const double rE = rho * igamma * (h + gm1 * v2h);
+  const double P = gm1 * (rE - rho * v2h);
+  return ((L.r < zero || L.E < tiny || L.P < tiny) ? 1 : 0) | ((R.r < zero || R.E < tiny || R.P < tiny) ? 2 : 0) |
+         ((P < tiny || rE < tiny) ? 4 : 0);
+}
+
+// the residual's Roe flux in either arithmetic
+__device__ __forceinline__ int roe_face(const dfl* QL, const dfl* QR, const dfl nx, const dfl ny, const dfl nz,
+                                        const dfl area, const dfl gamma, const dfl gm1, const dfl igamma,
+                                        const dfl igm1, dfl* flux) {
+  return roe_flux(QL, QR, nx, ny, nz, area, gamma, gm1, igamma, igm1, flux);
+}
+__device__ __forceinline__ int roe_face(const double* QL, const double* QR, const double nx, const double ny,
+                                        const double nz, const double area, const double gamma, const double gm1,
+                                        const double igamma, const double, double* flux) {
+  return roe_flux64(QL, QR, nx, ny, nz, area, gamma, gm1, igamma, flux);
 }
 
 // ComputeAuxiliaryVariables (ucs/compressible.tcc:1230) on a 10-wide FP64 record

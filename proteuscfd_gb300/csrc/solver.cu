@@ -1150,6 +1150,16 @@ __device__ __forceinline__ int kneecap5(S* f) {
   return bad;
 }
 
+// the same in FP64: one integer test of the exponents clears a finite flux
+template <>
+__device__ __forceinline__ int kneecap5<double>(double* f) {
+  if (!(not_finite(f[0]) | not_finite(f[1]) | not_finite(f[2]) | not_finite(f[3]) | not_finite(f[4]))) return 0;
+  int bad = 0;
+  for (int i = 0; i < NEQN; i++)
+    if (isnan(f[i])) { f[i] = 0.0; bad = 1; }
+  return bad;
+}
+
 // Kernel_Inviscid_Flux (:192) for one edge, stored as the flux leaving the
 // left node (k_edge_visc adds the viscous part).
 // MODE 0: plain evaluation.  MODE 1: also flags the nodes whose extrapolated
@@ -1215,7 +1225,7 @@ __global__ void __launch_bounds__(128) k_edge_flux(int nedge, const int2* __rest
     }
   }
   S f[NEQN];
-  int bad = roe_flux(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
+  int bad = roe_face(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
   if (MODE == 1 && kd.clip && ((clipflag[n.x] | clipflag[n.y]) & 2)) {
     // an endpoint had negative raw limiter values, which the clip sees
     // before they are clamped: test the states it would build
@@ -1323,7 +1333,7 @@ __global__ void __launch_bounds__(128) k_bedge_flux(int nbedge, const int2* __re
   S QL[NEQN], QR[NEQN], f[NEQN];
 #pragma unroll
   for (int t = 0; t < NEQN; t++) { QL[t] = qL[t]; QR[t] = qR[t]; }
-  roe_flux(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
+  roe_face(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
   if (kneecap5(f)) atomicAdd(&health[H_KNEECAP], 1ull);
   if (kd.viscous) {
     S Q0 = halve(qL[0] + qR[0]), Q1 = halve(qL[1] + qR[1]), Q2 = halve(qL[2] + qR[2]), Q3 = halve(qL[3] + qR[3]),

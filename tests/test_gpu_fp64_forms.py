@@ -1,0 +1,68 @@
+"""The FP64 residual kernels' reduced-instruction forms where their branches
+lie: the entropy fix of the acoustic waves and operands outside the range of
+the FP32 seeds, against the oracle."""
+import numpy as np
+import pytest
+
+from oracle_lib import OracleSpace
+from parity import assert_residual_close
+from proteuscfd_gb300 import SolutionSpace, cases
+
+pytestmark = pytest.mark.gpu
+
+
+def random_states(kind, nrows, seed):
+    """Rows of physical states: "sonic" around Mach 1 in random directions
+    (the acoustic entropy fix switches on and off), "jumps" with densities and
+    pressures over three decades."""
+    rng = np.random.default_rng(seed)
+    if kind == "sonic":
+        rho, p = 1.4 * rng.uniform(0.8, 1.2, nrows), rng.uniform(0.8, 1.2, nrows)
+        speed = np.sqrt(1.4 * p / rho) * rng.uniform(0.7, 1.3, nrows)
+    else:
+        rho, p = 10.0 ** rng.uniform(-2, 1, nrows), 10.0 ** rng.uniform(-2, 1, nrows)
+        speed = np.sqrt(1.4 * p / rho) * rng.uniform(0.0, 3.0, nrows)
+    d = rng.normal(size=(nrows, 3))
+    u = d / np.linalg.norm(d, axis=1, keepdims=True) * speed[:, None]
+    q = np.zeros((nrows, 10))
+    q[:, 0], q[:, 1:4] = rho, rho[:, None] * u
+    q[:, 4] = p / 0.4 + 0.5 * rho * speed ** 2
+    return cases.with_aux(q)
+
+
+@pytest.mark.parametrize("kind", ["sonic", "jumps"])
+@pytest.mark.parametrize("dims", [(9, 7, 6), (2, 2, 2)])
+def test_roe_flux_against_oracle(kind, dims):
+    """First-order Roe fluxes of every edge and half-edge.  A component is
+    formed with fewer than 200 roundings of terms no larger than 20 of its
+    magnitude at Mach 3: 200 * 20 * 2^-53 = 4.4e-13, within the 1e-12 bar."""
+    case = cases.euler_ramp(*dims, seed=4)
+    m = cases.build_mesh(case)
+    S = SolutionSpace(m, case.param)
+    O = OracleSpace(m, case.param)
+    q = random_states(kind, m.nnode + m.nbedge, 21)
+    S.set_state(q)
+    b, _ = S.compute_residuals()
+    bo, _, kc = O.residual(q)
+    assert kc == 0 and S.health()[0] == 0
+    assert_residual_close(b, bo, O.last_babs)
+
+
+@pytest.mark.parametrize("power", [-130, -40, 40, 120])
+def test_roe_flux_scales_with_the_state(power):
+    """The flux is linear in a common factor of density, momentum and energy.
+    Factors of 2^-130 and 2^120 put every reciprocal and root outside the
+    seeds' exponent range (2^-100 .. 2^100), so the plain operators run; a
+    power of two changes no other rounding.  Same bound as above."""
+    case = cases.euler_ramp(9, 7, 6, seed=4)
+    m = cases.build_mesh(case)
+    S = SolutionSpace(m, case.param)
+    O = OracleSpace(m, case.param)
+    q = random_states("jumps", m.nnode + m.nbedge, 22)
+    S.set_state(q)
+    b, _ = S.compute_residuals()
+    O.residual(q)
+    q[:, :5] *= 2.0 ** power
+    S.set_state(cases.with_aux(q))
+    bs, _ = S.compute_residuals()
+    assert_residual_close(bs * 2.0 ** -power, b, O.last_babs)
