@@ -440,8 +440,10 @@ __global__ void __launch_bounds__(128) k_jac_bedge_df(int nthreads, BedgeSlots s
   for (int t = 0; t < NVARS; t++) nQ0[t] = 0.0;
   if (bct == PCFD_BC_NOSLIP && bnrm[he] >= 0)
     for (int t = 0; t < NVARS; t++) nQ0[t] = q[(size_t)bnrm[he] * NVARS + t];
-  // the condition on the stored state, in FP64 as the boundary update does
-  if (!apply_bc(bk, bct, QL0, QR0, ba[he], btw[he], nQ0)) atomicAdd(&health[H_BADBC], 1ull);
+  // the condition on the stored state in FP64, in the generic forms: a
+  // difference in its last FP64 bit can move the 48-bit value it is rounded
+  // to, and 2^-48 over h = 1e-8 is 4e-7 of the block
+  if (!apply_bc<true>(bk, bct, QL0, QR0, ba[he], btw[he], nQ0)) atomicAdd(&health[H_BADBC], 1ull);
   const D4 a = ba[he];
   dfl QL[NVARS], QR[NVARS], nQ[NVARS], qinf[NVARS];
   for (int t = 0; t < NVARS; t++) {

@@ -1,12 +1,13 @@
 """The FP64 residual kernels' reduced-instruction forms where their branches
-lie: the entropy fix of the acoustic waves and operands outside the range of
-the FP32 seeds, against the oracle."""
+lie: the entropy fix of the acoustic waves, operands outside the range of the
+FP32 seeds, the characteristic conditions' regimes, against the oracle."""
 import numpy as np
 import pytest
 
 from oracle_lib import OracleSpace
 from parity import assert_residual_close
 from proteuscfd_gb300 import SolutionSpace, cases
+from proteuscfd_gb300 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +67,33 @@ def test_roe_flux_scales_with_the_state(power):
     S.set_state(cases.with_aux(q))
     bs, _ = S.compute_residuals()
     assert_residual_close(bs * 2.0 ** -power, b, O.last_babs)
+
+
+@pytest.mark.parametrize("mach", [0.0, 0.3, 0.999, 1.6])
+@pytest.mark.parametrize("noise", [0.0, 0.2])
+def test_boundary_forms_against_oracle(mach, noise):
+    """The far-field and slip-wall sub-iterations: flow into, out of, along
+    and (exactly) not through the faces, sub- and supersonic, and phantom
+    rows whose average with the node has no positive pressure.  Ten
+    sub-iterations of about 50 roundings of terms up to 5 of the result:
+    10 * 50 * 5 * 2^-53 = 2.8e-13, held to 1e-12 of the column's magnitude."""
+    case = cases.euler_ramp(9, 7, 6, seed=4)
+    p = case.param
+    p.mach = mach
+    p.bc_type = {1: N.BC_FARFIELD, 2: N.BC_FARFIELD, 3: N.BC_IMPERMEABLE_WALL, 4: N.BC_FARFIELD, 5: N.BC_SYMMETRY,
+                 6: N.BC_FARFIELD}
+    m = cases.build_mesh(case)
+    S = SolutionSpace(m, p)
+    O = OracleSpace(m, p)
+    q = cases.perturbed_state(S.qinf(), m.nnode + m.nbedge, 5, amp=noise)
+    if noise:
+        rng = np.random.default_rng(6)
+        far = np.flatnonzero(np.isin(m.bfactag, (1, 2, 4, 6)))
+        q[m.nnode + rng.choice(far, len(far) // 8, replace=False), 4] *= -3.0
+        q = cases.with_aux(q)
+    S.set_state(q)
+    S.update_bcs()
+    qg, qo = S.get_state(), O.update_bcs(q)
+    assert np.array_equal(np.isnan(qg), np.isnan(qo))
+    scale = np.maximum(np.nanmax(np.abs(qo[:, :7]), axis=0), 1e-300)
+    assert np.nanmax(np.abs(qg - qo)[:, :7] / scale) <= 1e-12
