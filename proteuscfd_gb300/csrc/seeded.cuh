@@ -24,6 +24,10 @@ namespace pcfd {
 __device__ __forceinline__ bool seed_range(double x) {
   return (unsigned)(__double2hiint(x) - ((1023 - 100) << 20)) < (200u << 20);
 }
+// |v| without the sign bit
+__device__ __forceinline__ double abs_bits(double v) {
+  return __hiloint2double(__double2hiint(v) & 0x7fffffff, __double2loint(v));
+}
 // FP32 value of a double in seed_range (truncated) and back (exact)
 __device__ __forceinline__ float seed_f32(double x) {
   const unsigned hi = (unsigned)__double2hiint(x) - ((1023u - 127u) << 20);
@@ -69,6 +73,15 @@ __device__ __forceinline__ double recip(double x) {
   return fma(y0, fma(e, e, e), y0);
 }
 
+// a / b within 0.5 ulp + 2^-20 ulp: the quotient's residual formed exactly
+__device__ __forceinline__ double quot(double a, double b) {
+  if (!seed_range(abs_bits(b)) || !(seed_range(abs_bits(a)) || abs_bits(a) == 0.0)) return a / b;
+  const double ra = recip(abs_bits(b));
+  const double r = __double2hiint(b) < 0 ? -ra : ra;
+  const double q = a * r;
+  return fma(fma(-b, q, a), r, q);
+}
+
 // sqrt(x) and *inv = 1 / sqrt(x), each within 1 ulp
 __device__ __forceinline__ double sqrt_inv(double x, double* inv) {
   if (!seed_range(x)) {
@@ -102,11 +115,11 @@ __device__ __forceinline__ long long order_key(double v) {
   const long long b = __double_as_longlong(v);
   return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
-__device__ __forceinline__ bool key_gt(double a, double b) { return order_key(a) > order_key(b); }
-// |v| without the sign bit
-__device__ __forceinline__ double abs_bits(double v) {
-  return __hiloint2double(__double2hiint(v) & 0x7fffffff, __double2loint(v));
+// the double of a key
+__device__ __forceinline__ double key_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
 }
+__device__ __forceinline__ bool key_gt(double a, double b) { return order_key(a) > order_key(b); }
 // infinite or NaN
 __device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
 

@@ -873,10 +873,6 @@ __device__ __forceinline__ double fma_s<double>(double a, double b, double c) { 
 // keys that order doubles as their values (sign bit flips the magnitude),
 // so the FP64 pipe the limiter is bound by does not spend two comparisons
 // per neighbour and equation on them; the double-float path compares values.
-__device__ __forceinline__ long long dkey(double v) {
-  const long long b = __double_as_longlong(v);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
 template <class S>
 __device__ __forceinline__ void bound_upd(S v, S& mn, S& mx, long long&, long long&) {
   mx = (mx > v) ? mx : v;
@@ -884,7 +880,7 @@ __device__ __forceinline__ void bound_upd(S v, S& mn, S& mx, long long&, long lo
 }
 template <>
 __device__ __forceinline__ void bound_upd<double>(double v, double& mn, double& mx, long long& kmn, long long& kmx) {
-  const long long kv = dkey(v);
+  const long long kv = order_key(v);
   if (!(kmx > kv)) { kmx = kv; mx = v; }
   if (!(kmn < kv)) { kmn = kv; mn = v; }
 }
@@ -1009,7 +1005,182 @@ __device__ __forceinline__ void limit_node(int i, int k0, int k1, const int* __r
 }
 
 // Standalone limiter (Limiter<T>::Compute after a separate gradient): the
-// neighbour bounds, then limit_node.
+// neighbour bounds, then limit_node (FP64 at chi = 0: limit_node64).
+// ---- the FP64 limiter at chi = 0 ------------------------------------------
+// The limiter of an equation is the smallest of its neighbours' values, so
+// only the neighbour that attains it needs FP64.  Each neighbour's u = 1 - r
+// is estimated in FP32 with a bound on its error, and the two largest are
+// kept; where the bounds leave the maximum to them, they (mostly the first
+// alone) are evaluated in FP64, elsewhere limit_exact runs over all
+// neighbours.  Per neighbour and equation FP64 then forms only the extrapolation (5 instructions, which the
+// edge pass reads anyway) where the full evaluation takes 15.  Limiter pass of
+// the 128x96x96 box with +-1 % noise: 2.546 ms before, 1.166 now; of a
+// 53x37x29 box with the plain Venkatakrishnan limiter 291 us before, 162 now.
+
+// dx of neighbour entry k, and grad.dx in the reference's rounding
+__device__ __forceinline__ double limit_gdx(int se, const double* __restrict__ eh, double g0, double g1, double g2) {
+  const double* hv = &eh[3 * (size_t)(se < 0 ? ~se : se)];
+  const bool flip = se >= 0;
+  return dot3_ref<double>(g0, flip ? -hv[0] : hv[0], g1, flip ? -hv[1] : hv[1], g2, flip ? -hv[2] : hv[2]);
+}
+
+// r of one neighbour in FP64 (as limit_node forms it)
+template <int LIM>
+__device__ __forceinline__ double limit_value(double q, double qmin, double qmax, double gdx, double ep2) {
+  const double Q = __dadd_rn(q, gdx);
+  const double DM = Q - q;
+  if (LIM == 3) {
+    const double DP = (Q > q ? qmax : qmin) - q;
+    const double C1 = fma(DP, DP, ep2);
+    return quot(fma(DM, DP + DP, C1), fma(DM, fma(2.0, DM, DP), C1));
+  }
+  double r = 1.0;
+  if (Q > q) r = quot(qmax - q, DM);
+  else if (Q < q) r = quot(qmin - q, DM);
+  if (LIM == 1) {
+    r = (r > 0.0) ? r : 0.0;
+    return (r < 1.0) ? r : 1.0;
+  }
+  return quot(r * r + 2.0 * r, r * r + r + 2.0);
+}
+
+// the smallest r over all neighbours, one equation
+template <int LIM>
+__device__ __noinline__ double limit_exact(int k0, int k1, const int* __restrict__ nedg,
+                                           const double* __restrict__ eh, double q, double qmin, double qmax,
+                                           double g0, double g1, double g2, double ep2) {
+  double v = 1.0;
+  for (int k = k0; k < k1; k++) {
+    const double r = limit_value<LIM>(q, qmin, qmax, limit_gdx(nedg[k], eh, g0, g1, g2), ep2);
+    if (r < v) v = r;
+  }
+  return v;
+}
+
+template <int LIM>
+__device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* __restrict__ nedg,
+                                             const double* __restrict__ eh, const double* __restrict__ vol, double K3,
+                                             const double* qi, const double* gi, const long long* kmn,
+                                             const long long* kmx, double* __restrict__ limraw,
+                                             double* __restrict__ lim, int* __restrict__ clipflag,
+                                             double* __restrict__ ext) {
+  const double ep2 = 6.0 * 3.141592653589793 * vol[i] * K3;
+  const float ep2f = est_f32(ep2);
+  const float inf = __int_as_float(0x7f800000);
+  float dpp[NEQN], dpm[NEQN], qe[NEQN];
+  // per equation: the two largest estimates with their error bounds and
+  // entries, and the upper bound v3 of all other entries
+  float u1[NEQN], m1[NEQN], u2[NEQN], m2[NEQN], v3[NEQN];
+  int e1[NEQN], e2[NEQN];
+  bool flat[NEQN];   // Venkatakrishnan: some neighbour's extrapolation leaves the value as it is (r = 3/4)
+  bool nil[NEQN];    // Barth: some neighbour's r is certainly 0
+  bool range[NEQN];  // operands FP32 can square
+#pragma unroll
+  for (int t = 0; t < NEQN; t++) {
+    dpp[t] = est_f32(key_value(kmx[t]) - qi[t]);
+    dpm[t] = est_f32(key_value(kmn[t]) - qi[t]);
+    qe[t] = fabsf(est_f32(qi[t]));
+    u1[t] = u2[t] = v3[t] = -inf;
+    m1[t] = m2[t] = 0.0f;
+    e1[t] = e2[t] = k0;
+    flat[t] = nil[t] = false;
+    range[t] = ep2f > 1.0e-30f && ep2f < 1.0e30f && qe[t] < 1.0e15f && fabsf(dpp[t]) < 1.0e15f &&
+               fabsf(dpm[t]) < 1.0e15f;
+  }
+  for (int k = k0; k < k1; k++) {
+    const int se = nedg[k];
+    const double* hv = &eh[3 * (size_t)(se < 0 ? ~se : se)];
+    double dx0 = hv[0], dx1 = hv[1], dx2 = hv[2];
+    if (se >= 0) { dx0 = -dx0; dx1 = -dx1; dx2 = -dx2; }
+    double* xo = ext ? &ext[(size_t)(se < 0 ? ~se : se) * (2 * NEQN) + (se < 0 ? 0 : NEQN)] : nullptr;
+#pragma unroll
+    for (int t = 0; t < NEQN; t++) {
+      const double gdx = dot3_ref<double>(gi[3 * t], dx0, gi[3 * t + 1], dx1, gi[3 * t + 2], dx2);
+      if (xo) xo[t] = gdx;
+      const float dm = est_f32(gdx);
+      const float dp = dm > 0.0f ? dpp[t] : dpm[t];
+      float u, m;
+      if (LIM == 3) {
+        // u = DM (2 DM - DP) / den.  Each operand is within 2^-22, den keeps
+        // at least 0.47 of its terms' magnitudes, so u is within 2.9e-6 a /
+        // den; the rounding of q + grad.dx moves DM by up to 2^-53 |q|
+        const float am = fabsf(dm), a = 2.0f * am + fabsf(dp);
+        const float rd = rcp_f32(dp * dp + ep2f + dm * (dp + 2.0f * dm));
+        u = dm * (2.0f * dm - dp) * rd;
+        m = (3.0e-6f * am * a + 4.0e-16f * qe[t] * (a + 2.0f * am)) * rd;
+        if (!(range[t] && am < 1.0e15f)) {
+          u = 0.0f;
+          m = inf;
+        }
+      } else {
+        // r is a function of DP / DM with a slope of at most 1, flat where the
+        // ratio is large, and the ratio is within 2^-20 of itself where the
+        // rounding of q + grad.dx is small against DM (3e-6 covers both)
+        const float am = fabsf(dm), tr = dp * rcp_f32(dm);
+        u = LIM == 1 ? 1.0f - fminf(fmaxf(tr, 0.0f), 1.0f) : (2.0f - tr) * rcp_f32(tr * tr + tr + 2.0f);
+        m = 3.0e-6f;
+        if (!(range[t] && am > 1.0e-9f * qe[t] && am > 1.0e-30f && am < 1.0e15f && fabsf(tr) < 1.0e15f)) {
+          u = 0.0f;
+          m = inf;
+        } else if (LIM == 1 && tr < -1.0e-5f) {
+          nil[t] = true;
+        }
+      }
+      if ((__double2hiint(gdx) & 0x7fffffff) == 0 && __double2loint(gdx) == 0) {
+        flat[t] = true;
+        u = -inf;
+        m = 0.0f;
+      }
+      if (u > u1[t]) {
+        v3[t] = fmaxf(v3[t], u2[t] + m2[t]);
+        u2[t] = u1[t];
+        m2[t] = m1[t];
+        e2[t] = e1[t];
+        u1[t] = u;
+        m1[t] = m;
+        e1[t] = k;
+      } else if (u > u2[t]) {
+        v3[t] = fmaxf(v3[t], u2[t] + m2[t]);
+        u2[t] = u;
+        m2[t] = m;
+        e2[t] = k;
+      } else {
+        v3[t] = fmaxf(v3[t], u + m);
+      }
+    }
+  }
+  int neg = 0;
+#pragma unroll
+  for (int t = 0; t < NEQN; t++) {
+    double v;
+    const float low = u1[t] - m1[t], second = u2[t] + m2[t];
+    if (LIM == 1 && nil[t]) {
+      v = 0.0;
+    } else if (fmaxf(fmaxf(u1[t] + m1[t], second), v3[t]) < 5.0e-17f) {
+      v = 1.0;  // no neighbour below 1 - 2^-54
+    } else if (v3[t] > fmaxf(low, 0.0f)) {
+      v = limit_exact<LIM>(k0, k1, nedg, eh, qi[t], key_value(kmn[t]), key_value(kmx[t]), gi[3 * t], gi[3 * t + 1],
+                           gi[3 * t + 2], ep2);
+    } else {
+      v = 1.0;
+      const double r1 = limit_value<LIM>(qi[t], key_value(kmn[t]), key_value(kmx[t]),
+                                         limit_gdx(nedg[e1[t]], eh, gi[3 * t], gi[3 * t + 1], gi[3 * t + 2]), ep2);
+      if (r1 < v) v = r1;
+      if (second > fmaxf(low, 0.0f)) {
+        const double r2 = limit_value<LIM>(qi[t], key_value(kmn[t]), key_value(kmx[t]),
+                                           limit_gdx(nedg[e2[t]], eh, gi[3 * t], gi[3 * t + 1], gi[3 * t + 2]), ep2);
+        if (r2 < v) v = r2;
+      }
+    }
+    if (LIM == 2 && flat[t] && 0.75 < v) v = 0.75;  // r at DM = 0
+    limraw[(size_t)i * NEQN + t] = v;
+    const bool below = __double2hiint(v) < 0 && v != 0.0;
+    if (below) neg = 1;
+    if (lim) lim[(size_t)i * NEQN + t] = below ? 0.0 : v;
+  }
+  clipflag[i] = neg ? 2 : 0;
+}
+
 template <class S, int LIM, bool CHI0>
 __global__ void __launch_bounds__(128) k_venkat(int nnode, const int* __restrict__ nptr,
                                                 const int* __restrict__ nedg, const int* __restrict__ nnbr,
@@ -1019,23 +1190,47 @@ __global__ void __launch_bounds__(128) k_venkat(int nnode, const int* __restrict
                                                 int* __restrict__ clipflag, S* __restrict__ ext) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nnode) return;
-  const S zero = Sc<S>::c(0.0);
-  S qi[NEQN], qmin[NEQN], qmax[NEQN], gi[NEQN * 3];
-  for (int t = 0; t < NEQN; t++) {
-    qi[t] = q[(size_t)i * NVARS + t];
-    qmin[t] = zero;
-    qmax[t] = zero;
+  if constexpr (std::is_same<S, double>::value && CHI0) {
+    double qi[NEQN], gi[NEQN * 3];
+    long long kmn[NEQN], kmx[NEQN];
+#pragma unroll
+    for (int t = 0; t < NEQN; t++) {
+      qi[t] = q[(size_t)i * NVARS + t];
+      kmn[t] = kmx[t] = 0;  // the key of +0.0, the bounds' start
+    }
+    const int k0 = nptr[i], k1 = nptr[i + 1];
+    for (int k = k0; k < k1; k++) {
+      const double* qj = &q[(size_t)nnbr[k] * NVARS];
+#pragma unroll
+      for (int t = 0; t < NEQN; t++) {
+        const long long kv = order_key(qj[t]);
+        if (kv > kmx[t]) kmx[t] = kv;
+        if (kv < kmn[t]) kmn[t] = kv;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < NEQN * 3; t++) gi[t] = grad[(size_t)i * NTERMS * 3 + t];
+    limit_node64<LIM>(i, k0, k1, nedg, eh, vol, K3, qi, gi, kmn, kmx, limraw, lim, clipflag, ext);
+    return;
+  } else {
+    const S zero = Sc<S>::c(0.0);
+    S qi[NEQN], qmin[NEQN], qmax[NEQN], gi[NEQN * 3];
+    for (int t = 0; t < NEQN; t++) {
+      qi[t] = q[(size_t)i * NVARS + t];
+      qmin[t] = zero;
+      qmax[t] = zero;
+    }
+    for (int t = 0; t < NEQN * 3; t++) gi[t] = grad[(size_t)i * NTERMS * 3 + t];
+    const int k0 = nptr[i], k1 = nptr[i + 1];
+    long long kmn[NEQN], kmx[NEQN];
+    for (int t = 0; t < NEQN; t++) kmn[t] = kmx[t] = 0;  // the key of +0.0, the bounds' start
+    for (int k = k0; k < k1; k++) {
+      const S* qj = &q[(size_t)nnbr[k] * NVARS];
+      for (int t = 0; t < NEQN; t++) bound_upd<S>(qj[t], qmin[t], qmax[t], kmn[t], kmx[t]);
+    }
+    limit_node<S, LIM, CHI0>(i, k0, k1, nedg, nnbr, q, eh, vol, chi_d, K3, qi, gi, qmin, qmax, limraw, lim, clipflag,
+                             ext);
   }
-  for (int t = 0; t < NEQN * 3; t++) gi[t] = grad[(size_t)i * NTERMS * 3 + t];
-  const int k0 = nptr[i], k1 = nptr[i + 1];
-  long long kmn[NEQN], kmx[NEQN];
-  for (int t = 0; t < NEQN; t++) kmn[t] = kmx[t] = 0;  // the key of +0.0, the bounds' start
-  for (int k = k0; k < k1; k++) {
-    const S* qj = &q[(size_t)nnbr[k] * NVARS];
-    for (int t = 0; t < NEQN; t++) bound_upd<S>(qj[t], qmin[t], qmax[t], kmn[t], kmx[t]);
-  }
-  limit_node<S, LIM, CHI0>(i, k0, k1, nedg, nnbr, q, eh, vol, chi_d, K3, qi, gi, qmin, qmax, limraw, lim, clipflag,
-                           ext);
 }
 
 // BadExtrapolation (ucs/compressible.tcc:1056)

@@ -1,6 +1,6 @@
 """The FP64 residual kernels' reduced-instruction forms where their branches
-lie: the entropy fix of the acoustic waves, operands outside the range of the
-FP32 seeds, the characteristic conditions' regimes, against the oracle."""
+lie - the entropy fix of the acoustic waves, operands outside the range of the
+FP32 seeds, the ends of the limiter's screening - against the oracle."""
 import numpy as np
 import pytest
 
@@ -97,3 +97,50 @@ def test_boundary_forms_against_oracle(mach, noise):
     assert np.array_equal(np.isnan(qg), np.isnan(qo))
     scale = np.maximum(np.nanmax(np.abs(qo[:, :7]), axis=0), 1e-300)
     assert np.nanmax(np.abs(qg - qo)[:, :7] / scale) <= 1e-12
+
+
+def limiter_state(kind, m, qinf, seed):
+    """States that end in each branch of the limiter's FP32 screening: "flat"
+    (every extrapolation leaves the value: no neighbour screens), "level"
+    (noise of 1e-15: every neighbour ties within its bound), "noise" (one
+    neighbour clears the others), "sheet" (equal values on two sides of a
+    plane: neighbours tie at equal ratios), "small" and "large" (operands FP32
+    cannot square)."""
+    rng = np.random.default_rng(seed)
+    n = m.nnode + m.nbedge
+    q = np.tile(qinf, (n, 1))
+    if kind == "sheet":
+        q[:, :5] *= np.where(rng.uniform(size=n) < 0.5, 0.9, 1.1)[:, None]
+    elif kind != "flat":
+        amp = {"level": 1e-15, "noise": 0.01, "small": 0.01, "large": 0.01}[kind]
+        q[:, :5] *= 1.0 + rng.uniform(-amp, amp, size=(n, 5))
+        q[:, 3] = 0.0
+    q[:, :5] *= {"small": 1e-19, "large": 1e19}.get(kind, 1.0)
+    return cases.with_aux(q)
+
+
+@pytest.mark.parametrize("kind", ["flat", "level", "noise", "sheet", "small", "large"])
+@pytest.mark.parametrize("limiter", [1, 2, 3])
+@pytest.mark.parametrize("dims", [(10, 8, 7), (3, 2, 2)])
+def test_limiter_screening_against_oracle(kind, limiter, dims):
+    """The limiter (with the pressure clip) of the GPU's own gradient: a value is one quotient of terms with fewer
+    than 20 roundings, conditioned by at most 1e3 where the extrapolated
+    change is above 1e-13 of the value: 20 * 1e3 * 2^-53 = 2.2e-12, held to
+    1e-11 (the level field's own bound: its ratios hang on the last bits, so
+    there only the range is checked)."""
+    case = cases.ns_flatplate(*dims, seed=5)
+    case.param.limiter = limiter
+    m = cases.build_mesh(case)
+    S = SolutionSpace(m, case.param)
+    O = OracleSpace(m, case.param)
+    q = limiter_state(kind, m, S.qinf(), 8)
+    S.set_state(q)
+    g = S.gradient()
+    lg = S.limiter()
+    if kind == "level":
+        assert np.all((lg >= 0.0) & (lg <= 1.0))
+        if limiter == 3:
+            assert np.abs(lg - 1.0).max() <= 1e-9  # eps^2 outweighs 1e-15 noise
+        return
+    lo, _ = O.limiter(q, g)
+    assert np.abs(lg - lo).max() <= 1e-11
