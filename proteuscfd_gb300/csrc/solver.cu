@@ -341,7 +341,7 @@ __device__ __forceinline__ S theta_ref(S t0, S t1, S t2, S t3, S ax, S ay, S az)
 template <>
 __device__ __forceinline__ double theta_ref<double>(double t0, double t1, double t2, double t3, double ax, double ay,
                                                     double az) {
-  return dot3_ref<double>(__ddiv_rn(t1, t0), ax, __ddiv_rn(t2, t0), ay, __ddiv_rn(t3, t0), az);
+  return dot3_ref<double>(quot(t1, t0), ax, quot(t2, t0), ay, quot(t3, t0), az);
 }
 
 constexpr int kBcSubits = 10;  // sub-iterations of the characteristic conditions
@@ -357,20 +357,20 @@ __device__ void bc_farfield(S gamma, const S* Qinf, const S* QL, S pi, S* QR, co
   for (int subit = 0; subit < nsub; subit++) {
     S t0 = (QL[0] + QR[0]) * half, t1 = (QL[1] + QR[1]) * half, t2 = (QL[2] + QR[2]) * half,
       t3 = (QL[3] + QR[3]) * half, t4 = (QL[4] + QR[4]) * half;
-    S it0 = one / t0;
+    S it0 = inv_s(t0);
     S theta = theta_ref<S>(t0, t1, t2, t3, ax, ay, az);
     S rhoi = QL[0];
-    S iri = one / QL[0];
+    S iri = inv_s(QL[0]);
     S ui = QL[1] * iri, vi = QL[2] * iri, wi = QL[3] * iri;
     S rhoinf = Qinf[0];
-    S uinf = Qinf[1] / Qinf[0], vinf = Qinf[2] / Qinf[0], winf = Qinf[3] / Qinf[0];
+    S uinf = div_s(Qinf[1], Qinf[0]), vinf = div_s(Qinf[2], Qinf[0]), winf = div_s(Qinf[3], Qinf[0]);
     S pinf = Qinf[6];
     S tu = t1 * it0, tv = t2 * it0, tw = t3 * it0;
     S pavg = gm1 * (t4 - t0 * (half * (tu * tu + tv * tv + tw * tw)));
     S rhoavg = t0;
-    S c2avg = gamma * (pavg / rhoavg);
-    S cavg = sqrt(c2avg);
-    S mach = fabs(theta / cavg);
+    S c2avg = gamma * div_s(pavg, rhoavg);
+    S cavg = sqrt_s(c2avg);
+    S mach = fabs(div_s(theta, cavg));
     if (theta == zero) {
       return;
     } else if (theta > zero && mach >= one) {
@@ -379,18 +379,18 @@ __device__ void bc_farfield(S gamma, const S* Qinf, const S* QL, S pi, S* QR, co
       for (int i = 0; i < NEQN; i++) QR[i] = Qinf[i];
     } else if (theta > zero && mach < one) {
       S pb = pinf;
-      S rhob = rhoi + (pb - pi) / c2avg;
-      S t = (pb - pi) / (rhoavg * cavg);
+      S rhob = rhoi + div_s(pb - pi, c2avg);
+      S t = div_s(pb - pi, rhoavg * cavg);
       S ub = ui - ax * t, vb = vi - ay * t, wb = wi - az * t;
       QR[0] = rhob; QR[1] = rhob * ub; QR[2] = rhob * vb; QR[3] = rhob * wb;
-      QR[4] = pb / gm1 + half * rhob * (ub * ub + vb * vb + wb * wb);
+      QR[4] = div_s(pb, gm1) + half * rhob * (ub * ub + vb * vb + wb * wb);
     } else if (theta < zero && mach < one) {
       S pb = half * (pinf + pi + rhoavg * cavg * (ax * (uinf - ui) + ay * (vinf - vi) + az * (winf - wi)));
-      S rhob = rhoinf + (pb - pinf) / c2avg;
-      S t = (pb - pinf) / (rhoavg * cavg);
+      S rhob = rhoinf + div_s(pb - pinf, c2avg);
+      S t = div_s(pb - pinf, rhoavg * cavg);
       S ub = uinf + ax * t, vb = vinf + ay * t, wb = winf + az * t;
       QR[0] = rhob; QR[1] = rhob * ub; QR[2] = rhob * vb; QR[3] = rhob * wb;
-      QR[4] = pb / gm1 + half * rhob * (ub * ub + vb * vb + wb * wb);
+      QR[4] = div_s(pb, gm1) + half * rhob * (ub * ub + vb * vb + wb * wb);
     } else {
       return;
     }
@@ -404,7 +404,7 @@ __device__ void bc_inviscid_wall(S gamma, int no_cvbc, const S* QL, S pi, S* QR,
   const S half = Sc<S>::c(0.5), one = Sc<S>::c(1.0), two = Sc<S>::c(2.0);
   const S gm1 = gamma - one;
   const S rhoi = QL[0];
-  const S iri = one / rhoi;
+  const S iri = inv_s(rhoi);
   const S ui = QL[1] * iri, vi = QL[2] * iri, wi = QL[3] * iri;
   if (no_cvbc) {
     S dot = QL[1] * ax + QL[2] * ay + QL[3] * az;
@@ -418,18 +418,18 @@ __device__ void bc_inviscid_wall(S gamma, int no_cvbc, const S* QL, S pi, S* QR,
   for (int subit = 0; subit < nsub; subit++) {
     S t0 = (QL[0] + QR[0]) * half, t1 = (QL[1] + QR[1]) * half, t2 = (QL[2] + QR[2]) * half,
       t3 = (QL[3] + QR[3]) * half, t4 = (QL[4] + QR[4]) * half;
-    S it0 = one / t0;
+    S it0 = inv_s(t0);
     S tu = t1 * it0, tv = t2 * it0, tw = t3 * it0;
     S rhoavg = t0;
     S pavg = gm1 * (t4 - t0 * (half * (tu * tu + tv * tv + tw * tw)));
-    S c2avg = gamma * (pavg / rhoavg);
-    S cavg = sqrt(c2avg);
+    S c2avg = gamma * div_s(pavg, rhoavg);
+    S cavg = sqrt_s(c2avg);
     S pb = pi + rhoavg * cavg * thetaL;
-    S rhob = rhoi + (pb - pi) / c2avg;
-    S t = (pb - pi) / (rhoavg * cavg);
+    S rhob = rhoi + div_s(pb - pi, c2avg);
+    S t = div_s(pb - pi, rhoavg * cavg);
     S ub = ui - ax * t, vb = vi - ay * t, wb = wi - az * t;
     QR[0] = rhob; QR[1] = rhob * ub; QR[2] = rhob * vb; QR[3] = rhob * wb;
-    QR[4] = pb / gm1 + half * rhob * (ub * ub + vb * vb + wb * wb);
+    QR[4] = div_s(pb, gm1) + half * rhob * (ub * ub + vb * vb + wb * wb);
   }
 }
 
@@ -444,15 +444,15 @@ __device__ __noinline__ void bc_inviscid_wall_rest(double gamma, const double* Q
   bc_inviscid_wall<double>(gamma, 0, QL, pi, QR, ax, ay, az, nsub);
 }
 
-// The FP64 forms.  A sub-iteration is one long FP64 dependency chain and its
+// The FP64 forms of all sub-iterations but the last, which runs in the generic
+// form: the state it ends in then rounds as that form's does (the iteration
+// before it enters through the wave speeds, multiplied by the pressure or
+// velocity step across the face).  A sub-iteration is one long FP64 dependency chain and its
 // instructions run at 2 per clock per SM, so it is written for few of them
 // (about 50 in the far field and 25 at the wall, 140 in the generic forms):
 // the average state is kept as the sum of both sides; one root of
 // gamma p rho = (rho c)^2 with its reciprocal (sqrt_inv) gives rho c, c^2 and
-// both quotients by them.  Boundary update of the 10x8x8 box (latency of the
-// chain) 235 us before, 106 now; of the 128x96x96 box 995 us before, 365 now.
-// The FP64 boundary Jacobian, which runs six of these a half-edge, 2.24 ms on
-// the 64x48x48 box before, 0.96 now.
+// both quotients by them.
 __device__ __forceinline__ void bc_farfield64(double gamma, const double* Qinf, const double* QL, double pi,
                                               double* QR, double ax, double ay, double az) {
   const double gm1 = gamma - 1.0, hgm1 = 0.5 * gm1, igm1 = recip(gm1);
@@ -461,7 +461,7 @@ __device__ __forceinline__ void bc_farfield64(double gamma, const double* Qinf, 
   const double rhoinf = Qinf[0], uinf = Qinf[1] * irinf, vinf = Qinf[2] * irinf, winf = Qinf[3] * irinf;
   const double pinf = Qinf[6], dpo = pinf - pi, psum = pinf + pi;
   const double ndu = fma(ax, uinf - ui, fma(ay, vinf - vi, az * (winf - wi)));
-  for (int subit = 0; subit < kBcSubits; subit++) {
+  for (int subit = 0; subit < kBcSubits - 1; subit++) {
     const double s0 = QL[0] + QR[0], s1 = QL[1] + QR[1], s2 = QL[2] + QR[2], s3 = QL[3] + QR[3], s4 = QL[4] + QR[4];
     const double is0 = recip(s0);
     const double tu = s1 * is0, tv = s2 * is0, tw = s3 * is0;
@@ -498,6 +498,7 @@ __device__ __forceinline__ void bc_farfield64(double gamma, const double* Qinf, 
     QR[3] = rb * wb;
     QR[4] = fma(pb, igm1, 0.5 * fma(QR[1], ub, fma(QR[2], vb, QR[3] * wb)));
   }
+  bc_farfield<double>(gamma, Qinf, QL, pi, QR, ax, ay, az, 1);
 }
 
 // Slip wall and symmetry.  The phantom velocity is the interior one less its
@@ -523,7 +524,7 @@ __device__ __forceinline__ void bc_inviscid_wall64(double gamma, const double* Q
     s4 = QL[4] + QR[4];
   }
   double pb = 0.0;
-  for (int subit = 0; subit < kBcSubits; subit++) {
+  for (int subit = 0; subit < kBcSubits - 1; subit++) {
     const double s0 = rhoi + rb, is0 = recip(s0);
     const double pavg = hgm1 * fma(-0.5 * msq, is0, s4);
     const double t0 = 0.5 * s0, a = gamma * pavg * t0;
@@ -547,6 +548,7 @@ __device__ __forceinline__ void bc_inviscid_wall64(double gamma, const double* Q
   QR[2] = rb * vb;
   QR[3] = rb * wb;
   QR[4] = fma(pb, igm1, rb * hub2);
+  bc_inviscid_wall<double>(gamma, 0, QL, pi, QR, ax, ay, az, 1);
 }
 
 // FP64 entry points of the boundary kernels
@@ -1004,8 +1006,6 @@ __device__ __forceinline__ void limit_node(int i, int k0, int k1, const int* __r
   clipflag[i] = neg ? 2 : 0;
 }
 
-// Standalone limiter (Limiter<T>::Compute after a separate gradient): the
-// neighbour bounds, then limit_node (FP64 at chi = 0: limit_node64).
 // ---- the FP64 limiter at chi = 0 ------------------------------------------
 // The limiter of an equation is the smallest of its neighbours' values, so
 // only the neighbour that attains it needs FP64.  Each neighbour's u = 1 - r
@@ -1181,6 +1181,8 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
   clipflag[i] = neg ? 2 : 0;
 }
 
+// Standalone limiter (Limiter<T>::Compute after a separate gradient): the
+// neighbour bounds, then limit_node (FP64 at chi = 0: limit_node64).
 template <class S, int LIM, bool CHI0>
 __global__ void __launch_bounds__(128) k_venkat(int nnode, const int* __restrict__ nptr,
                                                 const int* __restrict__ nedg, const int* __restrict__ nnbr,
@@ -1544,7 +1546,7 @@ __global__ void __launch_bounds__(128) k_edge_flux(int nedge, const int2* __rest
     }
   }
   S f[NEQN];
-  int bad = roe_face(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
+  int bad = roe_flux(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
   if (MODE == 1 && kd.clip && ((clipflag[n.x] | clipflag[n.y]) & 2)) {
     // an endpoint had negative raw limiter values, which the clip sees
     // before they are clamped: test the states it would build
@@ -1652,7 +1654,7 @@ __global__ void __launch_bounds__(128) k_bedge_flux(int nbedge, const int2* __re
   S QL[NEQN], QR[NEQN], f[NEQN];
 #pragma unroll
   for (int t = 0; t < NEQN; t++) { QL[t] = qL[t]; QR[t] = qR[t]; }
-  roe_face(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
+  roe_flux(QL, QR, a.x, a.y, a.z, a.w, k.gamma, k.gm1, k.igamma, k.igm1, f);
   if (kneecap5(f)) atomicAdd(&health[H_KNEECAP], 1ull);
   if (kd.viscous) {
     S Q0 = halve(qL[0] + qR[0]), Q1 = halve(qL[1] + qR[1]), Q2 = halve(qL[2] + qR[2]), Q3 = halve(qL[3] + qR[3]),
