@@ -22,8 +22,16 @@ template <>
 __device__ __forceinline__ __nv_bfloat16 to_store<__nv_bfloat16>(double v) { return __double2bfloat16(v); }
 
 __device__ __forceinline__ double ld_blk(const double* p) { return *p; }
-__device__ __forceinline__ double ld_blk(const float* p) { return (double)*p; }
-__device__ __forceinline__ double ld_blk(const __nv_bfloat16* p) { return (double)__bfloat162float(*p); }
+// an FP32 value as a double, exactly, on the integer pipes (the conversion
+// instruction runs on the FP64 pipe); zero, subnormal, infinite and NaN
+// values take the conversion
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return m == 0u ? __hiloint2double((int)b, 0) : (double)f;
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + ((1023u - 127u) << 20))), (int)(b << 29));
+}
+__device__ __forceinline__ double ld_blk(const float* p) { return widen(*p); }
+__device__ __forceinline__ double ld_blk(const __nv_bfloat16* p) { return widen(__bfloat162float(*p)); }
 __device__ __forceinline__ float ld_blkf(const double* p) { return (float)*p; }
 __device__ __forceinline__ float ld_blkf(const float* p) { return *p; }
 __device__ __forceinline__ float ld_blkf(const __nv_bfloat16* p) { return __bfloat162float(*p); }
@@ -40,14 +48,6 @@ __device__ __forceinline__ void numflux(const double* QL, const double* QR, cons
 // QL/QR are the nodal 10-wide records (their stored pressure is used, as
 // GetPressure reads it); aL/aR are the left/right blocks with the sign the
 // reference scatters them with.
-template <class R>
-__device__ void viscous_jacobian(const R* QL, const R* QR, const R* dx, R s2, R ax, R ay, R az, R aw, R gamma, R Pr,
-                                 R inv_retilde, R S, R* aL, R* aR) {
-  const R half = R(0.5), one = R(1.0), two = R(2.0);
-  R Q0 = half * (QL[0] + QR[0]), Q1 = half * (QL[1] + QR[1]), Q2 = half * (QL[2] + QR[2]),
-         Q3 = half * (QL[3] + QR[3]), Q4 = half * (QL[4] + QR[4]);
-  R gm1 = gamma - one;
-  R iQ0 = Den<R>(Q0).of(one);
 // Quotients by one denominator: FP64 shares the reciprocal and corrects each
 // quotient by its residual (rounded as the operator rounds), FP32 divides.
 template <class R>
@@ -70,6 +70,14 @@ struct Den<double> {
   }
 };
 
+template <class R>
+__device__ void viscous_jacobian(const R* QL, const R* QR, const R* dx, R s2, R ax, R ay, R az, R aw, R gamma, R Pr,
+                                 R inv_retilde, R S, R* aL, R* aR) {
+  const R half = R(0.5), one = R(1.0), two = R(2.0);
+  R Q0 = half * (QL[0] + QR[0]), Q1 = half * (QL[1] + QR[1]), Q2 = half * (QL[2] + QR[2]),
+         Q3 = half * (QL[3] + QR[3]), Q4 = half * (QL[4] + QR[4]);
+  R gm1 = gamma - one;
+  R iQ0 = Den<R>(Q0).of(one);
   R ua = Q1 * iQ0, va = Q2 * iQ0, wa = Q3 * iQ0;
   R Pa = gm1 * (Q4 - half * Q0 * (ua * ua + va * va + wa * wa));
   R Ta = gamma * Pa * iQ0;
@@ -81,6 +89,8 @@ struct Den<double> {
   R rhoR = QR[0], uR = nR.of(QR[1]), vR = nR.of(QR[2]), wR = nR.of(QR[3]), PR = QR[6];
   R u = half * (uL + uR), v = half * (vL + vR), w = half * (wL + wR);
   R DxL[3], DxR[3];
+  const Den<R> dL(rhoL * s2), dR(rhoR * s2);
+#pragma unroll
   for (int i = 0; i < 3; i++) {
     DxL[i] = dL.of(-dx[i]);
     DxR[i] = dR.of(dx[i]);
@@ -90,8 +100,6 @@ struct Den<double> {
   R c1 = -(Den<R>(Pr).of(mu) * cp);
 #pragma unroll
   for (int side = 0; side < 2; side++) {
-  const Den<R> dL(rhoL * s2), dR(rhoR * s2);
-#pragma unroll
     const R* D = side ? DxR : DxL;
     R* A = side ? aR : aL;
     const Den<R>& n = side ? nR : nL;
@@ -137,14 +145,6 @@ struct JacConst {
   int viscous;
 };
 
-// Kernel_NumJac (ucs/jacobian.tcc:254): one-sided finite differences of the
-// Roe flux (h = 1e-8, 11 flux evaluations per edge) into A(R,L) and A(L,R),
-// plus Kernel_Viscous_Jac (:734) when viscous.
-// q is the state the inviscid differences see (the state before the boundary
-// conditions: ComputeSpatialJacobian runs Kernel_NumJac before Bkernel_NumJac
-// applies them, ucs/jacobian.tcc:186-188); qv the state after them, which
-// the viscous blocks see (Kernel_Viscous_Jac runs after, :190-194).
-template <class T>
 // difference quotient of two double-float fluxes in the block type's
 // arithmetic (h = 1e-8, whose reciprocal 1e8 is exact in FP32)
 __device__ __forceinline__ double df_quot(dfl d, double) { return to_dbl(d) * 1.0e8; }
@@ -203,6 +203,14 @@ __device__ __forceinline__ void jac_columns(const S* QL, const S* QR, const JacF
   for (int i = 1; i < NEQN; i++) column(i, sL.ir, sR.ir, pr, pr);
 }
 
+// Kernel_NumJac (ucs/jacobian.tcc:254): one-sided finite differences of the
+// Roe flux (h = 1e-8, 11 flux evaluations per edge) into A(R,L) and A(L,R),
+// plus Kernel_Viscous_Jac (:734) when viscous.
+// q is the state the inviscid differences see (the state before the boundary
+// conditions: ComputeSpatialJacobian runs Kernel_NumJac before Bkernel_NumJac
+// applies them, ucs/jacobian.tcc:186-188); qv the state after them, which
+// the viscous blocks see (Kernel_Viscous_Jac runs after, :190-194).
+template <class T>
 __global__ void __launch_bounds__(128) k_jac_edge(int nedge, const int2* __restrict__ en, const D4* __restrict__ ea,
                                                   const double* __restrict__ eh, const double* __restrict__ q,
                                                   const double* __restrict__ qv,
@@ -1348,6 +1356,19 @@ __device__ __forceinline__ S max_eig(const S* QL, const S* QR, const V& a, S gam
   const S theta = u * a.x + v * a.y + w * a.z;
   const S e4 = fabs(theta + c), e5 = fabs(theta - c);
   return e4 > e5 ? e4 : e5;
+}
+
+// The FP64 form: |theta| + c, the larger of |theta + c| and |theta - c|, from
+// the face sums (the halves cancel in the velocity and in c^2), reciprocal
+// and root from FP32 seeds: 28 FP64 instructions a face against 60 (the
+// kernel keeps the FP64 pipe 85 % busy; 64x48x48 box: 94 us a call before, 68
+// now)
+__device__ __forceinline__ double max_eig(const double* QL, const double* QR, const D4& a, double gamma) {
+  const double s0 = QL[0] + QR[0], s1 = QL[1] + QR[1], s2 = QL[2] + QR[2], s3 = QL[3] + QR[3], s4 = QL[4] + QR[4];
+  const double ir = recip(s0);
+  const double u = s1 * ir, v = s2 * ir, w = s3 * ir;
+  const double c2 = (gamma * (gamma - 1.0)) * fma(-0.5, fma(s1, u, fma(s2, v, s3 * w)), s4) * ir;
+  return abs_bits(fma(u, a.x, fma(v, a.y, w * a.z))) + root(c2);
 }
 
 // ComputeTimesteps (ucs/timestep.tcc:7) with local time stepping:
