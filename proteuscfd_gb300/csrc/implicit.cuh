@@ -57,17 +57,8 @@ struct Den {
   __device__ __forceinline__ R of(R a) const { return a / b; }
 };
 template <>
-struct Den<double> {
-  double b, r;
-  bool ok;
-  __device__ __forceinline__ explicit Den(double x) : b(x), r(0.0), ok(seed_range(x)) {
-    if (ok) r = recip(x);
-  }
-  __device__ __forceinline__ double of(double a) const {
-    if (!ok || !(abs_bits(a) == 0.0 || seed_range(abs_bits(a)))) return a / b;
-    const double q = a * r;
-    return fma(fma(-b, q, a), r, q);
-  }
+struct Den<double> : Quot64 {
+  using Quot64::Quot64;
 };
 
 template <class R>

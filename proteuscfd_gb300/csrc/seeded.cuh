@@ -82,6 +82,21 @@ __device__ __forceinline__ double quot(double a, double b) {
   return fma(fma(-b, q, a), r, q);
 }
 
+// Quotients by one denominator: its reciprocal is shared and each quotient
+// corrected by its residual, 3 FP64 instructions apiece (rounded as quot's)
+struct Quot64 {
+  double b, r;
+  bool ok;
+  __device__ __forceinline__ explicit Quot64(double x) : b(x), r(0.0), ok(seed_range(x)) {
+    if (ok) r = recip(x);
+  }
+  __device__ __forceinline__ double of(double a) const {
+    if (!ok || !(abs_bits(a) == 0.0 || seed_range(abs_bits(a)))) return a / b;
+    const double q = a * r;
+    return fma(fma(-b, q, a), r, q);
+  }
+};
+
 // sqrt(x) and *inv = 1 / sqrt(x), each within 1 ulp
 __device__ __forceinline__ double sqrt_inv(double x, double* inv) {
   if (!seed_range(x)) {
