@@ -1207,11 +1207,12 @@ __device__ __forceinline__ void sgs_rows_staged(int nrows, const int4* __restric
 }
 
 // nsweeps sweeps in one cooperative launch through the staged pipeline
-// (k_sgs_sweep's phases and barriers); FP32 or FP64 blocks and vectors.
+// (k_sgs_sweep's phases and barriers), for FP64 colours of few rows (the rule
+// and both sides' times stand at k_sgs_sweep_rows).
 // Each warp starts the x-independent copies of its first two rows of the
 // next colour before the barrier, so they overlap the wait.
 template <class E>
-__global__ void __launch_bounds__(256, sizeof(E) == 8 ? 2 : 4) k_sgs_sweep_staged(int ncolor, const int* __restrict__ cptr,
+__global__ void __launch_bounds__(256, 2) k_sgs_sweep_staged(int ncolor, const int* __restrict__ cptr,
                                                           const int4* __restrict__ desc, const int* __restrict__ ja,
                                                           const E* __restrict__ M, const E* __restrict__ dinv,
                                                           const E* __restrict__ b, E* x, int nsweeps,
@@ -1238,6 +1239,201 @@ __global__ void __launch_bounds__(256, sizeof(E) == 8 ? 2 : 4) k_sgs_sweep_stage
         cp_async_wait<0>();
         return;
       }
+    }
+  }
+}
+
+// ---- block-SGS sweep, six rows a warp -------------------------------------
+// Lane l = 5 g + r (l < 30) owns matrix row r of the g-th of six block rows:
+// it forms that row's whole dot product with one accumulator per column, so no
+// partial sum crosses lanes.  A lane per coefficient needs a shuffle per block
+// and four shuffled additions per row, and its 14-neighbour block row cost 23
+// FP64 instructions (FP64 runs at 2 per clock per SM and was 65 % busy) or 432
+// instructions in FP32; here it is 14 and about 60.  The additions of a matrix
+// row and their order are those of the lane-per-coefficient form, so the
+// values are the same bit for bit.
+//
+// A block's coefficients are read straight into registers, five consecutive
+// ones a lane, two blocks ahead of the arithmetic (four ahead: 10 to 30 %
+// slower, one: 2 to 25 %); of x each lane reads one entry a block from L2
+// (other SMs write x between colours) and gets the other four by shuffles.
+// What does not depend on x (a step's descriptors, column ids, inverse
+// diagonal, right-hand side and first two blocks) is read before the barrier
+// that ends the previous colour.  One block of 24 (FP32) or 16 (FP64) warps
+// per SM: 152 blocks at the grid barrier where 608 or 304 stood, and 144 or 96
+// resident rows an SM where 32 or 16 were.  A block's warps fill up only to
+// kSweepSpread before another block joins: a colour of few rows is otherwise
+// held on a few SMs (FP64, 32x24x24: 338 us instead of 219).
+//
+// Two sweeps over flat-plate meshes, the staged kernel / this one:
+//   FP32: 12x10x8 117 / 110 us, 32x24x24 142 / 139, 64x48x48 384 / 299,
+//         128x96x96 2099 / 1828
+//   FP64: 12x10x8 146 / 193 us, 24x20x20 205 / 219, 28x24x20 218 / 219,
+//         32x24x24 239 / 219, 64x48x48 1012 / 641, 128x96x96 6353 / 3824
+// FP32 therefore always runs here.  In FP64 a lane's whole row is a chain of
+// 70 FP64 instructions at 64 clocks each, which a colour that the staged
+// kernel takes in one round of resident rows does not hide, so the rule is on
+// the rows per SM of the largest colour: 28x24x20
+// has 17, 24x20x20 12 and 32x24x24 23.
+constexpr int kSweepRows = 6;
+constexpr int kSweepSpread = 4;      // warps a block gets before another block is added
+constexpr int kSweepRowsPerSM = 17;  // FP64: rows per SM of the largest colour from which this kernel runs
+constexpr int kSweepChunk = 2;   // blocks read together
+constexpr int kSweepBlocks = 20; // blocks of a row in the unrolled part
+template <class E>
+struct SweepBlock {
+  static constexpr int warps = sizeof(E) == 8 ? 16 : 24;  // FP64 12 or 20: 3 to 7 % slower, FP32 20 or 32: 2 to 10 %
+};
+
+__device__ __forceinline__ float mul_sep(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_sep(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_sep(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_sep(double a, double b) { return __dadd_rn(a, b); }
+
+// A lane's block row: id (-1: none), first block, block count, and the column
+// ids of blocks r, r + 5, r + 10 and r + 15.
+struct SweepRow {
+  int i, b0, nb;
+  int j[kSweepBlocks / 5];
+};
+__device__ __forceinline__ SweepRow sweep_row(int step, int nrows, const int4* __restrict__ desc,
+                                              const int* __restrict__ ja, int g, int r) {
+  SweepRow s;
+  s.i = -1;
+  s.b0 = s.nb = 0;
+  const int k = step * kSweepRows + g;
+  if (g < kSweepRows && k < nrows) {
+    const int4 d = desc[k];
+    s.i = d.x;
+    s.b0 = d.y;
+    s.nb = d.z;
+  }
+#pragma unroll
+  for (int p = 0; p < kSweepBlocks / 5; p++) s.j[p] = 5 * p + r < s.nb ? ja[s.b0 + 5 * p + r] : 0;
+  return s;
+}
+
+// the lane's coefficients of the kSweepChunk blocks from k0 on (0 past the row's end)
+template <class E>
+__device__ __forceinline__ void sweep_blocks(const SweepRow& s, int k0, int r, const E* __restrict__ M,
+                                             E (&m)[kSweepChunk][5]) {
+#pragma unroll
+  for (int u = 0; u < kSweepChunk; u++) {
+    const E* p = M + (size_t)(s.b0 + k0 + u) * 25 + r * 5;
+#pragma unroll
+    for (int c = 0; c < 5; c++) m[u][c] = k0 + u < s.nb ? __ldg(p + c) : E(0);
+  }
+}
+// the lane's x entry of the same blocks
+template <class E>
+__device__ __forceinline__ void sweep_x(const SweepRow& s, int k0, int g, int r, const E* x, E (&xr)[kSweepChunk]) {
+#pragma unroll
+  for (int u = 0; u < kSweepChunk; u++) {
+    const int k = k0 + u;
+    const int j = __shfl_sync(0xffffffffu, s.j[k / 5], (5 * g + k % 5) & 31);
+    xr[u] = k < s.nb ? __ldcg(x + (size_t)j * 5 + r) : E(0);
+  }
+}
+
+// x-independent data of a lane's row besides the row itself
+template <class E>
+struct SweepConst {
+  E m[kSweepChunk][5], dinv[5], b;
+};
+template <class E>
+__device__ __forceinline__ void sweep_const(const SweepRow& s, int r, const E* __restrict__ M,
+                                            const E* __restrict__ dinv, const E* __restrict__ b, SweepConst<E>& q) {
+  sweep_blocks(s, 0, r, M, q.m);
+#pragma unroll
+  for (int c = 0; c < 5; c++) q.dinv[c] = s.i >= 0 ? __ldg(dinv + (size_t)s.i * 25 + r * 5 + c) : E(0);
+  q.b = s.i >= 0 ? __ldg(b + (size_t)s.i * 5 + r) : E(0);
+}
+
+// the row updates x_i = D_i^-1 (b_i - sum_j A_ij x_j) of a step
+template <class E>
+__device__ __forceinline__ void sweep_update(const SweepRow& s, SweepConst<E>& q, int g, int r,
+                                             const int* __restrict__ ja, const E* __restrict__ M, E* x) {
+  const unsigned full = 0xffffffffu;
+  const int nmax = __reduce_max_sync(full, s.nb);
+  E a[5] = {E(0), E(0), E(0), E(0), E(0)};
+  E mb[kSweepChunk][5], xr[2][kSweepChunk];
+  sweep_x(s, 0, g, r, x, xr[0]);
+#pragma unroll
+  for (int k = 0; k < kSweepBlocks / kSweepChunk; k++) {
+    if (k * kSweepChunk >= nmax) break;
+    E(&cur)[kSweepChunk][5] = (k & 1) ? mb : q.m;
+    E(&nxt)[kSweepChunk][5] = (k & 1) ? q.m : mb;
+    if (k + 1 < kSweepBlocks / kSweepChunk) {
+      if ((k + 1) * kSweepChunk < nmax) {
+        sweep_blocks(s, (k + 1) * kSweepChunk, r, M, nxt);
+        sweep_x(s, (k + 1) * kSweepChunk, g, r, x, xr[(k + 1) & 1]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSweepChunk; u++)
+#pragma unroll
+      for (int c = 0; c < 5; c++)
+        a[c] = fma(cur[u][c], __shfl_sync(full, xr[k & 1][u], (5 * g + c) & 31), a[c]);
+  }
+  for (int k = kSweepBlocks; k < s.nb; k++) {  // blocks past the unrolled part
+    const E* xu = x + (size_t)ja[s.b0 + k] * 5;
+    const E* mu = M + (size_t)(s.b0 + k) * 25 + r * 5;
+#pragma unroll
+    for (int c = 0; c < 5; c++) a[c] = fma(mu[c], __ldcg(xu + c), a[c]);
+  }
+  __syncwarp();
+  const E sum = add_sep(add_sep(add_sep(add_sep(a[0], a[1]), a[2]), a[3]), a[4]);
+  const E rhs = q.b - sum;
+  E v = E(0);
+#pragma unroll
+  for (int c = 0; c < 5; c++) {
+    const E t = mul_sep(q.dinv[c], __shfl_sync(full, rhs, (5 * g + c) & 31));
+    v = c == 0 ? t : add_sep(v, t);
+  }
+  if (s.i >= 0) x[(size_t)s.i * 5 + r] = v;
+}
+
+// nsweeps sweeps in one cooperative launch (the phases of k_sgs_sweep)
+template <class E>
+__global__ void __launch_bounds__(32 * SweepBlock<E>::warps, 1)
+    k_sgs_sweep_rows(int ncolor, const int* __restrict__ cptr, const int4* __restrict__ desc,
+                     const int* __restrict__ ja, const E* __restrict__ M, const E* __restrict__ dinv,
+                     const E* __restrict__ b, E* x, int nsweeps, unsigned int* __restrict__ bar,
+                     int* __restrict__ err) {
+  constexpr int NW = SweepBlock<E>::warps;
+  const int lane = threadIdx.x & 31, g = lane / 5, r = lane % 5;
+  const int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, W = gridDim.x * NW;
+  const int nphase = nsweeps * 2 * ncolor;
+  if (nphase <= 0) return;
+  int c = sgs_colour(0, ncolor);
+  int r0 = cptr[c], nr = cptr[c + 1] - r0;
+  SweepRow s;
+  SweepConst<E> q;
+  if (w * kSweepRows < nr) {
+    s = sweep_row(w, nr, desc + r0, ja, g, r);
+    sweep_const(s, r, M, dinv, b, q);
+  }
+  for (int p = 0; p < nphase;) {
+    for (int t = w; t * kSweepRows < nr; t += W) {
+      const bool more = (t + W) * kSweepRows < nr;
+      SweepRow sn;
+      if (more) sn = sweep_row(t + W, nr, desc + r0, ja, g, r);
+      sweep_update(s, q, g, r, ja, M, x);
+      if (more) {
+        s = sn;
+        sweep_const(s, r, M, dinv, b, q);
+      }
+    }
+    p = sgs_next_phase(p, nphase, ncolor);
+    if (p < nphase) {
+      c = sgs_colour(p, ncolor);
+      r0 = cptr[c];
+      nr = cptr[c + 1] - r0;
+      if (w * kSweepRows < nr) {
+        s = sweep_row(w, nr, desc + r0, ja, g, r);
+        sweep_const(s, r, M, dinv, b, q);
+      }
+      if (!grid_barrier(bar, gridDim.x, err)) return;
     }
   }
 }

@@ -2438,8 +2438,7 @@ int check_sweeps(Solver* s) {
   return PCFD_OK;
 }
 
-template <class E>
-int run_sweeps_staged(Solver* s, int nsweeps, const E* dinv, const E* b, E* x);
+int run_sweeps_f64(Solver* s, int nsweeps, const double* dinv, const double* b, double* x);
 
 template <class T>
 int run_sgs_t(Solver* s, int nsweeps, const double* b, double* x, double* dnorm) {
@@ -2463,10 +2462,10 @@ int run_sgs_t(Solver* s, int nsweeps, const double* b, double* x, double* dnorm)
     out = std::sqrt(v) / cnt;
     return PCFD_OK;
   };
-  // FP64 blocks and vectors run the staged kernel, mixed types the
+  // FP64 blocks and vectors choose by size, mixed types run the
   // register-staged one
   auto sweeps = [&](int k) -> int {
-    if (std::is_same<T, double>::value) return run_sweeps_staged<double>(s, k, s->d_dinv, b, x);
+    if (std::is_same<T, double>::value) return run_sweeps_f64(s, k, s->d_dinv, b, x);
     return run_sweeps<T, double>(s, k, s->d_dinv, b, x, xa);
   };
   int rc;
@@ -2528,10 +2527,43 @@ int run_sweeps_staged(Solver* s, int nsweeps, const E* dinv, const E* b, E* x) {
   return PCFD_OK;
 }
 
-// FP32 blocks and vectors: the staged kernel
+// nsweeps sweeps through the six-rows-a-warp kernel (cooperative; one block
+// per multiprocessor, none beyond what the largest colour fills kSweepSpread
+// warps of), blocks and vectors of type E
+template <class E>
+int run_sweeps_rows(Solver* s, int nsweeps, const E* dinv, const E* b, E* x) {
+  if (nsweeps <= 0) return PCFD_OK;
+  auto kern = k_sgs_sweep_rows<E>;
+  constexpr int nthr = 32 * SweepBlock<E>::warps;
+  int per_sm = 0;
+  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nthr, 0));
+  if (per_sm < 1) return set_err(PCFD_ERR_CUDA, "sgs: sweep kernel cannot be resident");
+  int maxrows = 1;
+  for (int c = 0; c < s->ncolor; c++) maxrows = std::max(maxrows, s->color_ptr[c + 1] - s->color_ptr[c]);
+  int grid = std::max(1, std::min(s->nsm, nblk(maxrows, kSweepRows * kSweepSpread)));
+  const E* M = (const E*)s->d_M;
+  int ncolor = s->ncolor;
+  void* args[] = {&ncolor, &s->d_cptr, &s->d_rowdesc, &s->d_ja, &M, &dinv, &b, &x, &nsweeps, &s->d_gbar, &s->d_sgs_err};
+  cudaError_t ce = cudaSuccess;
+  int rc = launch(s, T_SGS, [&] { ce = cudaLaunchCooperativeKernel((void*)kern, grid, nthr, args, 0, s->stream); });
+  if (rc) return rc;
+  if (ce != cudaSuccess) return set_err(PCFD_ERR_CUDA, std::string("sgs sweep launch: ") + cudaGetErrorString(ce));
+  return PCFD_OK;
+}
+
+// FP64 blocks and vectors: six rows a warp from kSweepRowsPerSM rows per
+// multiprocessor in the largest colour on, the staged kernel below
+int run_sweeps_f64(Solver* s, int nsweeps, const double* dinv, const double* b, double* x) {
+  int maxrows = 1;
+  for (int c = 0; c < s->ncolor; c++) maxrows = std::max(maxrows, s->color_ptr[c + 1] - s->color_ptr[c]);
+  if (maxrows < kSweepRowsPerSM * s->nsm) return run_sweeps_staged<double>(s, nsweeps, dinv, b, x);
+  return run_sweeps_rows<double>(s, nsweeps, dinv, b, x);
+}
+
+// FP32 blocks and vectors: six rows a warp at every size
 template <>
 int run_sgs_f_t<float>(Solver* s, int nsweeps, const float* b, float* x) {
-  return run_sweeps_staged<float>(s, nsweeps, s->d_dinvf, b, x);
+  return run_sweeps_rows<float>(s, nsweeps, s->d_dinvf, b, x);
 }
 
 int run_sgs_f(Solver* s, int nsweeps, const float* b, float* x) {
