@@ -2964,6 +2964,7 @@ struct Learned {
   double *y = nullptr, *sigma = nullptr, *vbuf = nullptr;  // [n][5], [1], [n][5]
   int* err = nullptr;
   int grid_red = 0;               // blocks of the grid-stride backward kernels
+  int grid_gather = 0;            // blocks of the gather's transpose
   int npb = 0;                    // nodes per block of the weight-gradient kernels
   std::vector<float*> sx, st;     // stored training pairs
 };
@@ -3027,10 +3028,14 @@ int lp_forward(Solver* s, bool train, double* z) {
   const int n = lp->n;
   const size_t nh = (size_t)n * LP_H;
   int rc = launch(s, T_LP_FWD, [&] {
-    k_lp_encode<<<nblk((long long)n * (LP_H / 2), 256), 256, 0, s->stream>>>(n, lp->x, lp->w, lp->h);
+    k_lp_encode<<<std::min(nblk(n, 8), 4 * s->nsm), 256, 0, s->stream>>>(n, lp->x, lp->w, lp->h);
   });
   if (rc) return rc;
-  const int tiles = nblk(n, LP_TILE);
+  // rows a block: the rule and both sides' times stand at k_lp_layer
+  const bool half = n <= 2 * LP_TILE * s->nsm;
+  const int tiles = nblk(n, half ? LP_TILE / 2 : LP_TILE);
+  const auto inner = half ? k_lp_layer<false, LP_TILE / 2> : k_lp_layer<false, LP_TILE>;
+  const auto last = half ? k_lp_layer<true, LP_TILE / 2> : k_lp_layer<true, LP_TILE>;
   for (int l = 0; l < LP_NL; l++) {
     const float* wl = lp->w + LP_OFF_L0 + l * LP_L_SIZE;
     const __nv_bfloat16* hin = lp->h + (train ? l : (l & 1)) * nh;
@@ -3039,11 +3044,11 @@ int lp_forward(Solver* s, bool train, double* z) {
     const __nv_bfloat16* img = lp->img_fwd + (size_t)l * LP_IMG;
     rc = launch(s, T_LP_FWD, [&] {
       if (l < LP_NL - 1)
-        k_lp_layer<false><<<tiles, LP_THREADS, LP_SMEM, s->stream>>>(
+        inner<<<tiles, LP_THREADS, LP_SMEM, s->stream>>>(
             n, s->d_nptr, s->d_nnbr, lp->ef, lp->invdeg, hin, wl, img, hout, mout, lp->w, nullptr, nullptr, nullptr,
             nullptr, lp->err);
       else
-        k_lp_layer<true><<<tiles, LP_THREADS, LP_SMEM, s->stream>>>(
+        last<<<tiles, LP_THREADS, LP_SMEM, s->stream>>>(
             n, s->d_nptr, s->d_nnbr, lp->ef, lp->invdeg, hin, wl, img, train ? hout : nullptr, mout, lp->w,
             train ? lp->out : nullptr, lp->y, lp->sigma, train ? nullptr : z, lp->err);
     });
@@ -3052,45 +3057,64 @@ int lp_forward(Solver* s, bool train, double* z) {
   return PCFD_OK;
 }
 
+// floats of nb partial arrays of len entries, rounded up to 16 bytes
+size_t lp_part_slice(int nb, int len) { return ((size_t)nb * len + 3) & ~(size_t)3; }
+
 // gradient of the loss against lp->t into lp->g (after lp_forward(train))
 int lp_backward(Solver* s) {
   Learned* lp = s->lp;
   const int n = lp->n;
   const size_t nh = (size_t)n * LP_H;
   const int tiles = nblk(n, LP_TILE);
-  const int gr = lp->grid_red;
+  const int gr = lp->grid_red, gg = lp->grid_gather;
   const int nwb = nblk(n, lp->npb);
-  auto reduce = [&](int nb, int len, float* dst) {
-    return launch(s, T_LP_BWD, [&] { k_lp_reduce<<<nblk(len, 256), 256, 0, s->stream>>>(nb, len, lp->part, dst); });
+  // each kernel's partials go to their own slice of part, all summed at the end
+  LpSegments sg;
+  int nseg = 0, blocks = 0;
+  float* part = lp->part;
+  auto segment = [&](int nb, int len, float* dst) {
+    sg.nblk[nseg] = nb;
+    sg.len[nseg] = len;
+    sg.first[nseg] = blocks;
+    sg.part[nseg] = part;
+    sg.grad[nseg++] = dst;
+    blocks += nblk(len, 32);
+    float* mine = part;
+    part += lp_part_slice(nb, len);
+    return mine;
   };
   int rc = launch(s, T_LP_BWD, [&] {
-    k_lp_dec_bwd<<<gr, 256, 0, s->stream>>>(n, lp->out, lp->t, lp->h + LP_NL * nh, lp->w, lp->dh, lp->part);
+    k_lp_dec_bwd<<<gr, 256, 0, s->stream>>>(n, lp->out, lp->t, lp->h + LP_NL * nh, lp->w, lp->dh,
+                                            segment(gr, LP_DEC_LEN, lp->g + LP_OFF_WOUT));
   });
-  if (rc || (rc = reduce(gr, LP_DEC_LEN, lp->g + LP_OFF_WOUT))) return rc;
+  if (rc) return rc;
   for (int l = LP_NL - 1; l >= 0; l--) {
     const float* wl = lp->w + LP_OFF_L0 + l * LP_L_SIZE;
     float* gl = lp->g + LP_OFF_L0 + l * LP_L_SIZE;
     rc = launch(s, T_LP_BWD, [&] {
       k_lp_layer_bwd<<<tiles, LP_THREADS, LP_SMEM, s->stream>>>(n, lp->dh, lp->h + (l + 1) * nh,
-                                                               lp->img_bwd + (size_t)l * LP_IMG, lp->dz, lp->dhs,
-                                                               lp->dm, lp->err);
+                                                               lp->img_bwd + (size_t)l * LP_IMG, lp->invdeg, lp->dz,
+                                                               lp->dhs, lp->dm, lp->err);
     });
     if (rc) return rc;
     rc = launch(s, T_LP_BWD, [&] {
-      k_lp_wgrad<<<nwb, 256, 0, s->stream>>>(n, lp->npb, lp->dz, lp->h + l * nh, lp->m + l * nh, lp->part);
+      k_lp_wgrad<<<nwb, 256, 0, s->stream>>>(n, lp->npb, lp->dz, lp->h + l * nh, lp->m + l * nh,
+                                             segment(nwb, LP_WG_LEN, gl + LP_L_WS));
     });
-    if (rc || (rc = reduce(nwb, LP_WG_LEN, gl + LP_L_WS))) return rc;
+    if (rc) return rc;
     rc = launch(s, T_LP_BWD, [&] {
-      k_lp_gather_bwd<<<gr, 256, 0, s->stream>>>(n, s->d_nptr, s->d_nnbr, lp->ef, lp->invdeg, lp->h + l * nh, wl,
-                                                lp->dhs, lp->dm, lp->dh, lp->part);
+      k_lp_gather_bwd<<<gg, 256, 0, s->stream>>>(n, s->d_nptr, s->d_nnbr, lp->ef, lp->h + l * nh, wl, lp->dhs, lp->dm,
+                                                lp->dh, segment(gg, LP_GB_LEN, gl + LP_L_WE));
     });
-    if (rc || (rc = reduce(gr, LP_GB_LEN, gl + LP_L_WE))) return rc;
+    if (rc) return rc;
   }
   rc = launch(s, T_LP_BWD, [&] {
-    k_lp_enc_bwd<<<nwb, 256, 0, s->stream>>>(n, lp->npb, lp->dh, lp->h, lp->x, lp->part);
+    k_lp_enc_bwd<<<nwb, 256, 0, s->stream>>>(n, lp->npb, lp->dh, lp->h, lp->x,
+                                             segment(nwb, LP_EB_LEN, lp->g + LP_OFF_WIN));
   });
-  if (rc || (rc = reduce(nwb, LP_EB_LEN, lp->g + LP_OFF_WIN))) return rc;
-  return PCFD_OK;
+  if (rc) return rc;
+  sg.first[nseg] = blocks;
+  return launch(s, T_LP_BWD, [&] { k_lp_reduce<<<blocks, 32 * LP_RED_RUNS, 0, s->stream>>>(sg); });
 }
 
 // sigma of lp->y, then the node features into lp->x
@@ -3158,10 +3182,11 @@ int lp_alloc(Solver* s) {
   lp->n = n;
   lp->nnz = 2LL * s->nedge;
   lp->grid_red = std::min(nblk(n, 8), 4 * 152);
-  lp->npb = std::max(256, nblk(n, 1216));
+  lp->npb = std::max(LP_WG_CHUNK, nblk(n, 2 * s->nsm));  // two blocks a multiprocessor
   const int nwb = nblk(n, lp->npb);
-  lp->part_len = std::max({(size_t)lp->grid_red * LP_DEC_LEN, (size_t)lp->grid_red * LP_GB_LEN,
-                           (size_t)nwb * LP_WG_LEN, (size_t)nwb * LP_EB_LEN});
+  lp->grid_gather = std::min(nblk(n, 16), LP_GB_SM * s->nsm);
+  lp->part_len = lp_part_slice(lp->grid_red, LP_DEC_LEN) + LP_NL * lp_part_slice(nwb, LP_WG_LEN) +
+                 LP_NL * lp_part_slice(lp->grid_gather, LP_GB_LEN) + lp_part_slice(nwb, LP_EB_LEN);
   const size_t nh = (size_t)n * LP_H;
   int rc;
   if ((rc = dalloc(&lp->ef, std::max<long long>(lp->nnz, 1)))) return rc;
@@ -3188,13 +3213,13 @@ int lp_alloc(Solver* s) {
   if ((rc = dalloc(&lp->err, 1))) return rc;
   CUDA_TRY(cudaMemsetAsync(lp->err, 0, sizeof(int), s->stream));
   CUDA_TRY(cudaMemsetAsync(lp->h, 0, (LP_NL + 1) * nh * sizeof(__nv_bfloat16), s->stream));
-  CUDA_TRY(cudaFuncSetAttribute(k_lp_layer<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM));
-  CUDA_TRY(cudaFuncSetAttribute(k_lp_layer<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM));
-  // three layer CTAs (3 x 51 KB) share a multiprocessor
-  CUDA_TRY(cudaFuncSetAttribute(k_lp_layer<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                (int)cudaSharedmemCarveoutMaxShared));
-  CUDA_TRY(cudaFuncSetAttribute(k_lp_layer<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                (int)cudaSharedmemCarveoutMaxShared));
+  // as many layer CTAs (51 KB each) on a multiprocessor as their registers allow
+  for (auto kern : {k_lp_layer<false, LP_TILE>, k_lp_layer<true, LP_TILE>, k_lp_layer<false, LP_TILE / 2>,
+                    k_lp_layer<true, LP_TILE / 2>}) {
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM));
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)cudaSharedmemCarveoutMaxShared));
+  }
   CUDA_TRY(cudaFuncSetAttribute(k_lp_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM));
   return launch(s, T_SETUP, [&] {
     k_lp_graph<<<nblk(n, 256), 256, 0, s->stream>>>(n, s->d_nptr, s->d_nedg, s->d_en, s->d_ea, s->d_xyz,
