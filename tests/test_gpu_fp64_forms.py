@@ -70,11 +70,12 @@ def test_roe_flux_scales_with_the_state(power):
 
 
 @pytest.mark.parametrize("mach", [0.0, 0.3, 0.999, 1.6])
-@pytest.mark.parametrize("noise", [0.0, 0.2])
+@pytest.mark.parametrize("noise", [0.0, 1e-9, 1e-3, 0.2])
 def test_boundary_forms_against_oracle(mach, noise):
     """The far-field and slip-wall sub-iterations: flow into, out of, along
     and (exactly) not through the faces, sub- and supersonic, and phantom
-    rows whose average with the node has no positive pressure.  Ten
+    rows whose average with the node has no positive pressure; sub-iterations
+    that reach their fixed point at once, after a few, or not.  Ten
     sub-iterations of about 50 roundings of terms up to 5 of the result:
     10 * 50 * 5 * 2^-53 = 2.8e-13, held to 1e-12 of the column's magnitude."""
     case = cases.euler_ramp(9, 7, 6, seed=4)
