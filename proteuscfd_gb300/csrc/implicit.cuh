@@ -161,7 +161,7 @@ struct JacFace {
 // separate evaluations.  The columns past the first run as
 // a loop, whose code stays in the instruction cache.  64x48x48 box: FP64 4.52 ms
 // before, 3.14 now (with the FP64 flux above); double-float 1.061 ms before,
-// 0.983 now.
+// 0.975 with this (0.887 with the blocks below).
 template <class S, class VR>
 __device__ __forceinline__ void jac_columns(const S* QL, const S* QR, const JacFace<S>& F, const S h, S* fS, VR* tL,
                                             VR* tR, unsigned long long* health) {
@@ -244,8 +244,13 @@ __global__ void __launch_bounds__(128) k_jac_edge(int nedge, const int2* __restr
 // ~1e-6 relative error: the Jacobian is only the Newton iteration matrix,
 // the residual (evaluated separately) decides the converged answer.  The
 // analytic viscous blocks stay FP64.
+// Issue (44 %) and instruction fetch bound it: a warp goes through its code
+// once an edge.  Blocks of 256, two an SM, measured 0.887 ms on the 64x48x48
+// box; 128 threads three or four an SM 0.975 and 1.048, 384 and 512 threads
+// 1.116 and 0.996.
+constexpr int kJacDfThreads = 256;
 template <class T>
-__global__ void __launch_bounds__(128, 3) k_jac_edge_df(int nedge, const int2* __restrict__ en,
+__global__ void __launch_bounds__(kJacDfThreads, 2) k_jac_edge_df(int nedge, const int2* __restrict__ en,
                                                      const D4* __restrict__ ea, const double* __restrict__ eh,
                                                      const double* __restrict__ q, const double* __restrict__ qv,
                                                      const int* __restrict__ pos_lr,

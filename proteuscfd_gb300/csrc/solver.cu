@@ -2336,7 +2336,7 @@ int run_jacobian_t(Solver* s) {
   const bool dfj = s->arith || !std::is_same<T, double>::value;
   int rc = launch(s, T_JAC_EDGE, [&] {
     if (dfj)
-      k_jac_edge_df<T><<<nblk(s->nedge, 128), 128, 0, s->stream>>>(s->nedge, s->d_en, s->d_ea, s->d_eh, s->d_qpre,
+      k_jac_edge_df<T><<<nblk(s->nedge, kJacDfThreads), kJacDfThreads, 0, s->stream>>>(s->nedge, s->d_en, s->d_ea, s->d_eh, s->d_qpre,
                                                                   s->d_q, s->d_pos_lr, s->d_pos_rl, jk, M,
                                                                   s->d_health);
     else
