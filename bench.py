@@ -693,8 +693,8 @@ def run_gb300(args, ws, rank, local, pg):
     # 128x96x96 box (profiles/residual_fp64_ns128.md), as a ratio to their
     # algorithmic bytes there, scaled to this box: the traffic grows with the
     # edges and nodes streamed
-    traffic_ratio = {"edge_flux": 1462.9 / 1393.9, "venkat_limiter": 1700.8 / 1155.1, "edge_viscous": 1498.7 / 1471.6,
-                     "lsq_gradient": 790.8 / 794.6, "residual_gather": 640.3 / 809.2}
+    traffic_ratio = {"edge_flux": 1460.4 / 1393.9, "venkat_limiter": 1654.5 / 1155.1, "edge_viscous": 1495.5 / 1471.6,
+                     "lsq_gradient": 788.0 / 794.6, "residual_gather": 614.5 / 809.2}
     traffic = alg_bytes * traffic_ratio[top] if top in traffic_ratio else None
     peak, peak_kind = peaks()
     # The FP64 kernels are bound by the FP64 pipe (2 FP64 instructions per
@@ -703,7 +703,7 @@ def run_gb300(args, ws, rank, local, pg):
     # (sm__inst_executed_pipe_fp64 x 32, profiles/residual_fp64_ns128.md);
     # achieved = those instructions over the kernel's event-timed launch,
     # peak = 2 x SMs x the median SM clock sampled during the timed region.
-    fp64_inst = {"edge_flux": (257.0, 0.0), "venkat_limiter": (0.0, 1145.0), "edge_viscous": (152.0, 0.0),
+    fp64_inst = {"edge_flux": (162.7, 0.0), "venkat_limiter": (0.0, 483.8), "edge_viscous": (118.0, 0.0),
                  "lsq_gradient": (0.0, 506.0), "residual_gather": (0.0, 184.0)}
     nsm = torch.cuda.get_device_properties(local).multi_processor_count
     sm_mhz = clk.summary().get("sm_mhz") or 0.0
@@ -795,7 +795,7 @@ def run_gb300(args, ws, rank, local, pg):
                     "ms": spmv_ms, "bytes": spmv_bytes, "achieved_gbs": spmv_bytes / (spmv_ms * 1e-3) / 1e9,
                     "peak_gbs": peak, "frac": spmv_bytes / (spmv_ms * 1e-3) / 1e9 / peak if peak else None}
 
-    # the block-SGS sweep (k_sgs_sweep_staged, one cooperative launch per
+    # the block-SGS sweep (k_sgs_sweep_rows, one cooperative launch per
     # call): the mixed solver's FP32 preconditioner sweep on the FP32 matrix,
     # then the FP64 arm's 10 FP64 sweeps on the FP64 matrix.  Algorithmic
     # bytes per sweep: the matrix twice (forward and backward pass) as in the
@@ -812,7 +812,7 @@ def run_gb300(args, ws, rank, local, pg):
     S.bench_sgs(1, 10, fp32=False)
     nrep64 = max(2, args.steps // 5)
     sgs64_ms = S.bench_sgs(nrep64, 10, fp32=False) / (10 * nrep64)
-    line["sgs"] = {"what": "block-SGS sweep (forward + backward, k_sgs_sweep_staged) on this box's %d-block "
+    line["sgs"] = {"what": "block-SGS sweep (forward + backward, k_sgs_sweep_rows) on this box's %d-block "
                            "matrix, vectors resident; ms per sweep" % nb,
                    "fp32": {"ms": sgs32_ms, "bytes": sgs_bytes(4),
                             "achieved_gbs": sgs_bytes(4) / (sgs32_ms * 1e-3) / 1e9,
