@@ -1518,8 +1518,10 @@ __device__ __forceinline__ int kneecap5<double>(double* f) {
 // the MUSCL correction is grad.dx alone (bit-identical to the general form).
 // EXT (chi = 0): both ends' corrections come from ext, as the limiter pass
 // formed them from the same gradient, instead of the gradient gathers.
+// Double-float: 128 registers a thread, four blocks an SM (161 and three
+// blocks: 96x72x64 box 250 us, 223 now; blocks of 256 two an SM 232).
 template <class S, int MODE, bool CHI0, bool EXT>
-__global__ void __launch_bounds__(128) k_edge_flux(int nedge, const int2* __restrict__ en,
+__global__ void __launch_bounds__(128, std::is_same<S, double>::value ? 0 : 4) k_edge_flux(int nedge, const int2* __restrict__ en,
                                                    const typename V4<S>::type* __restrict__ ea,
                                                    const S* __restrict__ eh, const S* __restrict__ q,
                                                    const S* __restrict__ grad, const S* __restrict__ lim, FluxConst kd,
