@@ -25,6 +25,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -574,7 +575,10 @@ __device__ __forceinline__ double transport_fit(const double (*fit)[6], int nfit
   return exp(c[2] * t.logT + t.q1.of(c[3]) + t.q2.of(c[4]) + c[5]) * conv;
 }
 
-// the molecular-weight factors of Wilke's rule, once per handle
+// the molecular-weight factors of Wilke's rule, once per handle: one block, a
+// thread per pair of species
+constexpr int kChemWilkePairs = PCFD_CHEM_MAX_SPECIES * PCFD_CHEM_MAX_SPECIES;
+static_assert(kChemWilkePairs <= 1024, "a block holds every pair of species");
 __global__ void k_chem_wilke(const pcfd_chem_model* __restrict__ gm, ChemDerived* __restrict__ gd) {
   const int i = threadIdx.x / PCFD_CHEM_MAX_SPECIES, j = threadIdx.x % PCFD_CHEM_MAX_SPECIES;
   if (i >= gm->nspecies || j >= gm->nspecies) return;
@@ -1620,21 +1624,27 @@ PCFD_API int pcfd_chem_create(const pcfd_chem_model* model, pcfd_chem_t* out) {
   }
   ChemHandle* c = new ChemHandle();
   std::memcpy(&c->host, model, sizeof(pcfd_chem_model));
+  // The uploads go on the handle's stream: it does not wait for the legacy
+  // stream, on which a copy from pageable memory may still be under way when
+  // cudaMemcpy returns, and k_chem_wilke reads one array and completes the other.
   cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e == cudaSuccess) e = cudaMalloc(&c->dev, sizeof(pcfd_chem_model));
-  if (e == cudaSuccess) e = cudaMemcpy(c->dev, model, sizeof(pcfd_chem_model), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c->dev, &c->host, sizeof(pcfd_chem_model), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
-    static thread_local ChemDerived d;
-    derive(model, d);
+    const std::unique_ptr<ChemDerived> d(new ChemDerived);  // kept until the copy is done
+    derive(model, *d);
     e = cudaMalloc(&c->dder, sizeof(ChemDerived));
-    if (e == cudaSuccess) e = cudaMemcpy(c->dder, &d, sizeof(ChemDerived), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(c->dder, d.get(), sizeof(ChemDerived), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
-      k_chem_wilke<<<1, 256, 0, c->stream>>>(c->dev, c->dder);
+      k_chem_wilke<<<1, kChemWilkePairs, 0, c->stream>>>(c->dev, c->dder);
       e = cudaGetLastError();
-      if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     }
+    const cudaError_t done = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = done;
   }
   if (e != cudaSuccess) {
     int rc = cuda_fail(e, "pcfd_chem_create");
@@ -1970,9 +1980,10 @@ PCFD_API int pcfd_chem_attach_mesh(pcfd_chem_t h, const pcfd_mesh_view* m) {
   c->nnode = c->nedge = c->nbedge = 0;
   const int ns = c->host.nspecies, neqn = ns + 4;
   const size_t nv = 6 + 3 * (size_t)ns;
+  // on the handle's stream, whose kernels read the arrays (pcfd_chem_create)
   auto up = [&](void** dst, const void* src, size_t bytes) -> cudaError_t {
     cudaError_t e = cudaMalloc(dst, bytes > 0 ? bytes : 16);
-    if (e == cudaSuccess && bytes > 0) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && bytes > 0) e = cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
     return e;
   };
   cudaError_t e = cudaSuccess;
@@ -2000,8 +2011,9 @@ PCFD_API int pcfd_chem_attach_mesh(pcfd_chem_t h, const pcfd_mesh_view* m) {
       k_chem_lsq<<<CHEM_GRID(nn)>>>(nn, c->d_en, c->d_nptr, c->d_nedg, c->d_xyz, c->d_sw, c->d_lsq);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   }
+  const cudaError_t done = cudaStreamSynchronize(c->stream);  // before the host arrays go
+  if (e == cudaSuccess) e = done;
   if (e != cudaSuccess) return cuda_fail(e, "pcfd_chem_attach_mesh");
   c->nnode = nn;
   c->nedge = ne;
