@@ -1038,10 +1038,27 @@ __device__ __forceinline__ void limit_node(int i, int k0, int k1, const int* __r
 // is estimated in FP32 with a bound on its error, and the two largest are
 // kept; where the bounds leave the maximum to them, they (mostly the first
 // alone) are evaluated in FP64, elsewhere limit_exact runs over all
-// neighbours.  Per neighbour and equation FP64 then forms only the extrapolation (5 instructions, which the
-// edge pass reads anyway) where the full evaluation takes 15.  Limiter pass of
-// the 128x96x96 box with +-1 % noise: 2.546 ms before, 1.166 now; of a
-// 53x37x29 box with the plain Venkatakrishnan limiter 291 us before, 162 now.
+// neighbours.  Per neighbour and equation FP64 then forms only the
+// extrapolation (5 instructions, which the edge pass reads anyway) where the
+// full evaluation takes 15.
+//
+// A neighbour whose r is 1 or more for certain counts for nothing: most are,
+// the bounds starting at 0 (DP = -q for a falling extrapolation).  Limiters 1
+// and 2 have no eps^2 to drown the rounding of q + grad.dx, so where that
+// counts the change is formed as it is rounded (2 more instructions), and
+// neighbours with the same change as the first, or whose bound is the value
+// itself, are told from near ties by exact comparisons.  Without these three
+// limit_exact ran almost everywhere in a stream quiet to 1e-12 (limiter 3) or
+// 1e-6 (2), and for 1 at any amplitude.
+// us a pass of the full evaluation over all neighbours / this one:
+//   53x37x29 box, noise of 1e-16, 1e-15, 1e-12, 1e-6, 1e-2 of the values
+//     1 Barth     126/121  222/130  193/130  193/110  192/93
+//     2 plain     201/128  334/151  274/142  273/120  274/98
+//     3 modified  137/72   137/72   137/73   138/79   137/75
+//   128x96x96 box
+//     1           2198/1569  4130/1697  3438/1680  3440/1406  3443/1353
+//     2           3716/1613  6262/1861  4854/1765  4845/1489  4856/1430
+//     3           2546/1016  2546/1013  2546/1016  2546/1174  2546/1165
 
 // dx of neighbour entry k, and grad.dx in the reference's rounding
 __device__ __forceinline__ double limit_gdx(int se, const double* __restrict__ eh, double g0, double g1, double g2) {
@@ -1097,21 +1114,25 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
   // per equation: the two largest estimates with their error bounds and
   // entries, and the upper bound v3 of all other entries
   float u1[NEQN], m1[NEQN], u2[NEQN], m2[NEQN], v3[NEQN];
+  float d1[NEQN];    // the first's change where an FP32 value holds it exactly, else 0
   int e1[NEQN], e2[NEQN];
   bool flat[NEQN];   // Venkatakrishnan: some neighbour's extrapolation leaves the value as it is (r = 3/4)
   bool nil[NEQN];    // Barth: some neighbour's r is certainly 0
   bool range[NEQN];  // operands FP32 can square
 #pragma unroll
   for (int t = 0; t < NEQN; t++) {
-    dpp[t] = est_f32(key_value(kmx[t]) - qi[t]);
-    dpm[t] = est_f32(key_value(kmn[t]) - qi[t]);
+    const double DPP = key_value(kmx[t]) - qi[t], DPM = key_value(kmn[t]) - qi[t];
+    dpp[t] = est_f32(DPP);
+    dpm[t] = est_f32(DPM);
     qe[t] = fabsf(est_f32(qi[t]));
     u1[t] = u2[t] = v3[t] = -inf;
     m1[t] = m2[t] = 0.0f;
     e1[t] = e2[t] = k0;
     flat[t] = nil[t] = false;
     range[t] = ep2f > 1.0e-30f && ep2f < 1.0e30f && qe[t] < 1.0e15f && fabsf(dpp[t]) < 1.0e15f &&
-               fabsf(dpm[t]) < 1.0e15f;
+               fabsf(dpm[t]) < 1.0e15f &&
+               (LIM == 3 || ((dpp[t] != 0.0f || DPP == 0.0) && (dpm[t] != 0.0f || DPM == 0.0)));
+    d1[t] = 0.0f;
   }
   for (int k = k0; k < k1; k++) {
     const int se = nedg[k];
@@ -1123,14 +1144,28 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
     for (int t = 0; t < NEQN; t++) {
       const double gdx = dot3_ref<double>(gi[3 * t], dx0, gi[3 * t + 1], dx1, gi[3 * t + 2], dx2);
       if (xo) xo[t] = gdx;
-      const float dm = est_f32(gdx);
+      float dm = est_f32(gdx);
+      // gdx is zero: the extrapolation leaves the value as it is
+      bool still = (__double2hiint(gdx) & 0x7fffffff) == 0 && __double2loint(gdx) == 0;
+      bool twin = false;  // the same change as the first's, so the same r
+      float de = 0.0f;
+      if (LIM != 3 && !still && !(fabsf(dm) > 1.0e-9f * qe[t])) {
+        // a change so small that the rounding of q + grad.dx counts in the
+        // ratio: the change as it is rounded
+        const double DM = __dadd_rn(qi[t], gdx) - qi[t];
+        still = DM == 0.0;
+        dm = est_f32(DM);
+        if ((__double2loint(DM) & 0x1fffffff) == 0) de = dm;  // exactly
+        twin = !still && de != 0.0f && de == d1[t];
+      }
       const float dp = dm > 0.0f ? dpp[t] : dpm[t];
+      const float am = fabsf(dm), ap = fabsf(dp);
       float u, m;
       if (LIM == 3) {
         // u = DM (2 DM - DP) / den.  Each operand is within 2^-22, den keeps
         // at least 0.47 of its terms' magnitudes, so u is within 2.9e-6 a /
         // den; the rounding of q + grad.dx moves DM by up to 2^-53 |q|
-        const float am = fabsf(dm), a = 2.0f * am + fabsf(dp);
+        const float a = 2.0f * am + ap;
         const float rd = rcp_f32(dp * dp + ep2f + dm * (dp + 2.0f * dm));
         u = dm * (2.0f * dm - dp) * rd;
         m = (3.0e-6f * am * a + 4.0e-16f * qe[t] * (a + 2.0f * am)) * rd;
@@ -1140,20 +1175,28 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
         }
       } else {
         // r is a function of DP / DM with a slope of at most 1, flat where the
-        // ratio is large, and the ratio is within 2^-20 of itself where the
-        // rounding of q + grad.dx is small against DM (3e-6 covers both)
-        const float am = fabsf(dm), tr = dp * rcp_f32(dm);
+        // ratio is large, and the ratio is within 2^-20 of itself (3e-6 covers
+        // the rounding of q + grad.dx, below 1.2e-7 of a change above 1e-9 |q|)
+        const float tr = dp * rcp_f32(dm);
         u = LIM == 1 ? 1.0f - fminf(fmaxf(tr, 0.0f), 1.0f) : (2.0f - tr) * rcp_f32(tr * tr + tr + 2.0f);
         m = 3.0e-6f;
-        if (!(range[t] && am > 1.0e-9f * qe[t] && am > 1.0e-30f && am < 1.0e15f && fabsf(tr) < 1.0e15f)) {
+        if (!(range[t] && am > 1.0e-30f && am < 1.0e15f && fabsf(tr) < 1.0e15f)) {
           u = 0.0f;
           m = inf;
+        } else if (dp == 0.0f) {  // r is 0
+          if (LIM == 1) nil[t] = true;
+          u = 1.0f;
+          m = 0.0f;
         } else if (LIM == 1 && tr < -1.0e-5f) {
           nil[t] = true;
         }
       }
-      if ((__double2hiint(gdx) & 0x7fffffff) == 0 && __double2loint(gdx) == 0) {
-        flat[t] = true;
+      // an allowed change of the same sign that is certainly as large as the
+      // extrapolated one (Barth) or twice it (the others): r is at least 1
+      const bool free = dm * dp > 0.0f &&
+                        ap > (LIM == 1 ? 1.00001f : 2.00001f) * am + (LIM == 3 ? 4.0e-16f * qe[t] : 0.0f);
+      if (still) flat[t] = true;
+      if (still || free || twin) {
         u = -inf;
         m = 0.0f;
       }
@@ -1165,6 +1208,7 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
         u1[t] = u;
         m1[t] = m;
         e1[t] = k;
+        d1[t] = de;
       } else if (u > u2[t]) {
         v3[t] = fmaxf(v3[t], u2[t] + m2[t]);
         u2[t] = u;
