@@ -1275,6 +1275,14 @@ __global__ void __launch_bounds__(256, 2) k_sgs_sweep_staged(int ncolor, const i
 //         128x96x96 2099 / 1828
 //   FP64: 12x10x8 146 / 193 us, 24x20x20 205 / 219, 28x24x20 218 / 219,
 //         32x24x24 239 / 219, 64x48x48 1012 / 641, 128x96x96 6353 / 3824
+// A row of more than kSweepBlocks blocks goes through the unrolled part again,
+// with its next column ids read one part ahead.  Unstructured meshes have
+// such rows in every colour (2 to 8 % of a Delaunay mesh's); summed one block
+// at a time past the first 20, they held up every phase.  Two sweeps over
+// Delaunay meshes of 24^3 and 56^3 jittered points, the staged kernel / one
+// block at a time / this:
+//   FP32: 457 / 621 / 353 us and 1247 / 1533 / 815
+//   FP64: the staged kernel 535 and 2104 / 2048 / 1684
 // FP32 therefore always runs here.  In FP64 a lane's whole row is a chain of
 // 70 FP64 instructions at 64 clocks each, which a colour that the staged
 // kernel takes in one round of resident rows does not hide, so the rule is on
@@ -1284,7 +1292,7 @@ constexpr int kSweepRows = 6;
 constexpr int kSweepSpread = 4;      // warps a block gets before another block is added
 constexpr int kSweepRowsPerSM = 17;  // FP64: rows per SM of the largest colour from which this kernel runs
 constexpr int kSweepChunk = 2;   // blocks read together
-constexpr int kSweepBlocks = 20; // blocks of a row in the unrolled part
+constexpr int kSweepBlocks = 20; // blocks of a row in the unrolled part, a multiple of 5 and twice kSweepChunk
 template <class E>
 struct SweepBlock {
   static constexpr int warps = sizeof(E) == 8 ? 16 : 24;  // FP64 12 or 20: 3 to 7 % slower, FP32 20 or 32: 2 to 10 %
@@ -1329,14 +1337,15 @@ __device__ __forceinline__ void sweep_blocks(const SweepRow& s, int k0, int r, c
     for (int c = 0; c < 5; c++) m[u][c] = k0 + u < s.nb ? __ldg(p + c) : E(0);
   }
 }
-// the lane's x entry of the same blocks
+// the lane's x entry of the same blocks, whose column ids are those of blocks
+// kj, kj + 1, .. of j
 template <class E>
-__device__ __forceinline__ void sweep_x(const SweepRow& s, int k0, int g, int r, const E* x, E (&xr)[kSweepChunk]) {
+__device__ __forceinline__ void sweep_x(const SweepRow& s, const int (&j)[kSweepBlocks / 5], int kj, int k0, int g,
+                                        int r, const E* x, E (&xr)[kSweepChunk]) {
 #pragma unroll
   for (int u = 0; u < kSweepChunk; u++) {
-    const int k = k0 + u;
-    const int j = __shfl_sync(0xffffffffu, s.j[k / 5], (5 * g + k % 5) & 31);
-    xr[u] = k < s.nb ? __ldcg(x + (size_t)j * 5 + r) : E(0);
+    const int id = __shfl_sync(0xffffffffu, j[(kj + u) / 5], (5 * g + (kj + u) % 5) & 31);
+    xr[u] = k0 + u < s.nb ? __ldcg(x + (size_t)id * 5 + r) : E(0);
   }
 }
 
@@ -1362,29 +1371,38 @@ __device__ __forceinline__ void sweep_update(const SweepRow& s, SweepConst<E>& q
   const int nmax = __reduce_max_sync(full, s.nb);
   E a[5] = {E(0), E(0), E(0), E(0), E(0)};
   E mb[kSweepChunk][5], xr[2][kSweepChunk];
-  sweep_x(s, 0, g, r, x, xr[0]);
+  int j[kSweepBlocks / 5];
 #pragma unroll
-  for (int k = 0; k < kSweepBlocks / kSweepChunk; k++) {
-    if (k * kSweepChunk >= nmax) break;
-    E(&cur)[kSweepChunk][5] = (k & 1) ? mb : q.m;
-    E(&nxt)[kSweepChunk][5] = (k & 1) ? q.m : mb;
-    if (k + 1 < kSweepBlocks / kSweepChunk) {
-      if ((k + 1) * kSweepChunk < nmax) {
-        sweep_blocks(s, (k + 1) * kSweepChunk, r, M, nxt);
-        sweep_x(s, (k + 1) * kSweepChunk, g, r, x, xr[(k + 1) & 1]);
+  for (int p = 0; p < kSweepBlocks / 5; p++) j[p] = s.j[p];
+  sweep_x(s, j, 0, 0, g, r, x, xr[0]);
+  for (int base = 0; base < nmax; base += kSweepBlocks) {
+    int jn[kSweepBlocks / 5];
+    if (base + kSweepBlocks < nmax) {
+#pragma unroll
+      for (int p = 0; p < kSweepBlocks / 5; p++) {
+        const int k = base + kSweepBlocks + 5 * p + r;
+        jn[p] = k < s.nb ? ja[s.b0 + k] : 0;
       }
     }
 #pragma unroll
-    for (int u = 0; u < kSweepChunk; u++)
+    for (int k = 0; k < kSweepBlocks / kSweepChunk; k++) {
+      if (base + k * kSweepChunk >= nmax) break;
+      E(&cur)[kSweepChunk][5] = (k & 1) ? mb : q.m;
+      E(&nxt)[kSweepChunk][5] = (k & 1) ? q.m : mb;
+      const int kn = base + (k + 1) * kSweepChunk;
+      if (kn < nmax) {
+        sweep_blocks(s, kn, r, M, nxt);
+        if (k + 1 < kSweepBlocks / kSweepChunk) sweep_x(s, j, (k + 1) * kSweepChunk, kn, g, r, x, xr[(k + 1) & 1]);
+        else sweep_x(s, jn, 0, kn, g, r, x, xr[(k + 1) & 1]);
+      }
 #pragma unroll
-      for (int c = 0; c < 5; c++)
-        a[c] = fma(cur[u][c], __shfl_sync(full, xr[k & 1][u], (5 * g + c) & 31), a[c]);
-  }
-  for (int k = kSweepBlocks; k < s.nb; k++) {  // blocks past the unrolled part
-    const E* xu = x + (size_t)ja[s.b0 + k] * 5;
-    const E* mu = M + (size_t)(s.b0 + k) * 25 + r * 5;
+      for (int u = 0; u < kSweepChunk; u++)
 #pragma unroll
-    for (int c = 0; c < 5; c++) a[c] = fma(mu[c], __ldcg(xu + c), a[c]);
+        for (int c = 0; c < 5; c++)
+          a[c] = fma(cur[u][c], __shfl_sync(full, xr[k & 1][u], (5 * g + c) & 31), a[c]);
+    }
+#pragma unroll
+    for (int p = 0; p < kSweepBlocks / 5; p++) j[p] = jn[p];
   }
   __syncwarp();
   const E sum = add_sep(add_sep(add_sep(add_sep(a[0], a[1]), a[2]), a[3]), a[4]);
