@@ -873,7 +873,10 @@ __device__ int fr_hllc(const ChemDerived& d, int ns, const pcfd_chem_ref& ref, c
 // (the kernel keeps the FP64 pipe 91 % busy).  With the divisions by one
 // denominator sharing its reciprocal, the 96x64x64 box's edge pass takes
 // 1.49 ms and this one 0.19, where the edge pass took 3.59.  Used where the
-// faces name each record twice or more on average (fewer: record_c2h).
+// faces name records more often than there are (names_repeat); fluxes of a
+// million records through faces that name 0.5, 0.8, 1, 1.2, 2 and 14 of them a
+// record, formed per face / here: 327/494 us, 512/581, 628/636, 745/690,
+// 1225/919, 8283/4278.
 __global__ void __launch_bounds__(128) k_chem_c2h(long long nrec, const pcfd_chem_model* __restrict__ gm,
                                                   const ChemDerived* __restrict__ gd, pcfd_chem_ref ref,
                                                   const double* __restrict__ q, double2* __restrict__ c2h) {
@@ -884,8 +887,7 @@ __global__ void __launch_bounds__(128) k_chem_c2h(long long nrec, const pcfd_che
   c2h[p] = make_double2(fr_c2(*gd, ns, ref, Q, Q[ns + 3]), fr_Ht(*gd, ns, ref, Q));
 }
 
-// a face's values of one record: stored, or formed here (c2h null) where the
-// faces name fewer records than there are
+// a face's values of one record: stored, or formed here (c2h null)
 __device__ __forceinline__ double2 record_c2h(const ChemDerived& d, int ns, const pcfd_chem_ref& ref, const double* Q,
                                               const double2* __restrict__ c2h, int rec) {
   if (c2h) return c2h[rec];
@@ -1574,16 +1576,29 @@ int node_call(ChemHandle* c, long long n, int dev, const double* const (&in)[NIN
   return PCFD_OK;
 }
 
-// the per-record part of the first-order flux for nrec records
-int run_c2h(ChemHandle* c, long long nrec, const pcfd_chem_ref& r, const double* q) {
+// whether nface faces of two records name records more often than there are
+bool names_repeat(long long nrec, long long nface) { return nrec < 2 * nface; }
+
+// The buffer of nrec per-record values, null where the device has no room for
+// it: the faces then form the values themselves, to the same bits.
+double2* ensure_c2h(ChemHandle* c, long long nrec) {
   if (c->c2h_cap < (size_t)nrec) {
     cudaFree(c->d_c2h);
     c->d_c2h = nullptr;
     c->c2h_cap = 0;
-    CHEM_TRY(cudaMalloc(&c->d_c2h, (size_t)nrec * sizeof(double2)), "chem buffers");
-    c->c2h_cap = (size_t)nrec;
+    if (cudaMalloc(&c->d_c2h, (size_t)nrec * sizeof(double2)) == cudaSuccess) {
+      c->c2h_cap = (size_t)nrec;
+    } else {
+      c->d_c2h = nullptr;
+      cudaGetLastError();
+    }
   }
-  k_chem_c2h<<<(unsigned)((nrec + 127) / 128), 128, 0, c->stream>>>(nrec, c->dev, c->dder, r, q, c->d_c2h);
+  return c->d_c2h;
+}
+
+// the per-record part of the first-order flux for nrec records into c2h
+int run_c2h(ChemHandle* c, long long nrec, const pcfd_chem_ref& r, const double* q, double2* c2h) {
+  k_chem_c2h<<<(unsigned)((nrec + 127) / 128), 128, 0, c->stream>>>(nrec, c->dev, c->dder, r, q, c2h);
   CHEM_TRY(cudaGetLastError(), "k_chem_c2h launch");
   return PCFD_OK;
 }
@@ -1908,10 +1923,10 @@ PCFD_API int pcfd_chem_hllc_flux(pcfd_chem_t h, const pcfd_chem_ref* ref, const 
   }
   const pcfd_chem_ref r = *ref;
   const pcfd_chem_flux_opts oo = *o;
-  const bool per_record = nnode < 2 * nedge;
-  if (per_record)
-    if (int rc = run_c2h(c, nnode, r, dq)) return rc;
-  k_chem_hllc<<<CHEM_GRID(nedge)>>>(nedge, nnode, c->dev, c->dder, r, oo, dq, per_record ? c->d_c2h : nullptr, de, da, df, c->d_count);
+  double2* c2h = names_repeat(nnode, nedge) ? ensure_c2h(c, nnode) : nullptr;
+  if (c2h)
+    if (int rc = run_c2h(c, nnode, r, dq, c2h)) return rc;
+  k_chem_hllc<<<CHEM_GRID(nedge)>>>(nedge, nnode, c->dev, c->dder, r, oo, dq, c2h, de, da, df, c->d_count);
   CHEM_TRY(cudaGetLastError(), "k_chem_hllc launch");
   if (!dev)
     CHEM_TRY(cudaMemcpyAsync(flux, df, (size_t)nedge * (ns + 4) * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
@@ -2015,6 +2030,7 @@ PCFD_API int pcfd_chem_attach_mesh(pcfd_chem_t h, const pcfd_mesh_view* m) {
   const cudaError_t done = cudaStreamSynchronize(c->stream);  // before the host arrays go
   if (e == cudaSuccess) e = done;
   if (e != cudaSuccess) return cuda_fail(e, "pcfd_chem_attach_mesh");
+  if (names_repeat(ntot, ne + nb)) ensure_c2h(c, ntot);
   c->nnode = nn;
   c->nedge = ne;
   c->nbedge = nb;
@@ -2246,10 +2262,10 @@ PCFD_API int pcfd_chem_residual(pcfd_chem_t h, const pcfd_chem_ref* ref, const p
   CHEM_TRY(cudaMemsetAsync(c->d_count, 0, sizeof(long long), c->stream), "chem count");
   const pcfd_chem_ref r = *ref;
   const pcfd_chem_flux_opts oo = *o;
-  const bool per_record = nn + nb < 2 * (ne + nb);
-  if (per_record)
-    if (int rc = run_c2h(c, nn + nb, r, dq)) return rc;
-  const double2* c2h = per_record ? c->d_c2h : nullptr;
+  // allocated with the mesh (or not, where there was no room)
+  double2* c2h = names_repeat(nn + nb, ne + nb) && c->c2h_cap >= (size_t)(nn + nb) ? c->d_c2h : nullptr;
+  if (c2h)
+    if (int rc = run_c2h(c, nn + nb, r, dq, c2h)) return rc;
   if (ne > 0) {
     k_chem_hllc<<<CHEM_GRID(ne)>>>(ne, nn + nb, c->dev, c->dder, r, oo, dq, c2h, c->d_en, c->d_ea, c->d_ef,
                                    c->d_count);
