@@ -1923,11 +1923,15 @@ int dalloc(T** p, size_t n) {
   return PCFD_OK;
 }
 
+// a new device array with h's values, on the handle's stream st: it does not
+// wait for the legacy stream, on which a copy from pageable memory may still
+// be under way when cudaMemcpy returns
 template <class T>
-int dput(T** p, const T* h, size_t n) {
+int dput(cudaStream_t st, T** p, const T* h, size_t n) {
   int rc = dalloc(p, n);
-  if (rc) return rc;
-  if (n) CUDA_TRY(cudaMemcpy(*p, h, n * sizeof(T), cudaMemcpyHostToDevice));
+  if (rc || n == 0) return rc;
+  CUDA_TRY(cudaMemcpyAsync(*p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
   return PCFD_OK;
 }
 
@@ -2503,8 +2507,8 @@ int check_sweeps(Solver* s) {
   int e = 0;
   CUDA_TRY(cudaMemcpy(&e, s->d_sgs_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e) {
-    CUDA_TRY(cudaMemset(s->d_sgs_err, 0, sizeof(int)));
-    CUDA_TRY(cudaMemset(s->d_gbar, 0, 2 * sizeof(unsigned int)));
+    CUDA_TRY(cudaMemsetAsync(s->d_sgs_err, 0, sizeof(int), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_gbar, 0, 2 * sizeof(unsigned int), s->stream));
     return set_err(PCFD_ERR_CUDA, "sgs: a sweep's grid barrier timed out");
   }
   return PCFD_OK;
@@ -3490,16 +3494,16 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
     ba[k] = D4{a[0], a[1], a[2], a[3]};
   }
 
-  TRY(dput(&s->d_en, en.data(), ne));
-  TRY(dput(&s->d_ea, ea.data(), ne));
-  TRY(dput(&s->d_bn, bn.data(), nb));
-  TRY(dput(&s->d_ba, ba.data(), nb));
-  TRY(dput(&s->d_bbc, bbc.data(), nb));
-  TRY(dput(&s->d_btw, btw.data(), nb));
-  TRY(dput(&s->d_bfactag, m->bfactag, nb));
-  TRY(dput(&s->d_bnrm, bnrm.data(), nb));
-  TRY(dput(&s->d_xyz, m->xyz, 3 * nn));
-  TRY(dput(&s->d_vol, m->vol, nn));
+  TRY(dput(s->stream, &s->d_en, en.data(), ne));
+  TRY(dput(s->stream, &s->d_ea, ea.data(), ne));
+  TRY(dput(s->stream, &s->d_bn, bn.data(), nb));
+  TRY(dput(s->stream, &s->d_ba, ba.data(), nb));
+  TRY(dput(s->stream, &s->d_bbc, bbc.data(), nb));
+  TRY(dput(s->stream, &s->d_btw, btw.data(), nb));
+  TRY(dput(s->stream, &s->d_bfactag, m->bfactag, nb));
+  TRY(dput(s->stream, &s->d_bnrm, bnrm.data(), nb));
+  TRY(dput(s->stream, &s->d_xyz, m->xyz, 3 * nn));
+  TRY(dput(s->stream, &s->d_vol, m->vol, nn));
   {
     // mean edge length and mean dual volume, summed in index order (the
     // learned preconditioner's feature scales)
@@ -3514,23 +3518,23 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
     s->lp_lmean = ne > 0 ? ls / ne : 1.0;
     s->lp_vmean = nn > 0 ? vs / nn : 1.0;
   }
-  TRY(dput(&s->d_nptr, nptr.data(), nn + 1));
-  TRY(dput(&s->d_nedg, nedg.data(), 2 * ne));
-  TRY(dput(&s->d_nnbr, nnbr.data(), 2 * ne));
-  TRY(dput(&s->d_bptr, bptr.data(), nn + 1));
-  TRY(dput(&s->d_bhe, bhe.data(), nb));
-  TRY(dput(&s->d_bgnode, gnode.data(), gnode.size()));
-  TRY(dput(&s->d_bgptr, gptr.data(), gptr.size()));
-  TRY(dput(&s->d_bghe, bghe_list.data(), bghe_list.size()));
+  TRY(dput(s->stream, &s->d_nptr, nptr.data(), nn + 1));
+  TRY(dput(s->stream, &s->d_nedg, nedg.data(), 2 * ne));
+  TRY(dput(s->stream, &s->d_nnbr, nnbr.data(), 2 * ne));
+  TRY(dput(s->stream, &s->d_bptr, bptr.data(), nn + 1));
+  TRY(dput(s->stream, &s->d_bhe, bhe.data(), nb));
+  TRY(dput(s->stream, &s->d_bgnode, gnode.data(), gnode.size()));
+  TRY(dput(s->stream, &s->d_bgptr, gptr.data(), gptr.size()));
+  TRY(dput(s->stream, &s->d_bghe, bghe_list.data(), bghe_list.size()));
   {
     std::vector<int> slot(bghe_list.size());
     for (size_t g = 0; g < gnode.size(); g++)
       for (int p = gptr[g]; p < gptr[g + 1]; p++) slot[p] = (int)g;
     s->nbgslot = (int)slot.size();
-    TRY(dput(&s->d_bgslot, slot.data(), slot.size()));
+    TRY(dput(s->stream, &s->d_bgslot, slot.data(), slot.size()));
     TRY(dalloc(&s->d_bgqr, std::max<size_t>(slot.size(), 1) * NVARS));
   }
-  TRY(dput(&s->d_bind, bind.data(), bind.size()));
+  TRY(dput(s->stream, &s->d_bind, bind.data(), bind.size()));
   TRY(dalloc(&s->d_clipflag, (size_t)nn));
   TRY(dalloc(&s->d_limraw, (size_t)nn * NEQN));
   TRY(dalloc(&s->d_clipany, 1));
@@ -3557,8 +3561,8 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
   }
   double* d_sw = nullptr;
   double* d_qinf = nullptr;
-  TRY(dput(&d_sw, m->sw, 6 * nn));
-  TRY(dput(&d_qinf, s->qinf, NVARS));
+  TRY(dput(s->stream, &d_sw, m->sw, 6 * nn));
+  TRY(dput(s->stream, &d_qinf, s->qinf, NVARS));
   TRY(launch(s, T_SETUP, [&] {
     k_lsq_weights<<<nblk(nn, 128), 128, 0, s->stream>>>(s->nnode, s->d_nptr, s->d_nnbr, s->d_xyz, d_sw, s->d_lsq);
   }));
@@ -3579,7 +3583,9 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
   // the limiter starts at 1.0 (OFF), as the Limiter constructor leaves it
   {
     std::vector<double> ones((size_t)nn * NEQN, 1.0);
-    if (cudaMemcpy(s->d_lim, ones.data(), ones.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (cudaMemcpyAsync(s->d_lim, ones.data(), ones.size() * sizeof(double), cudaMemcpyHostToDevice, s->stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(s->stream) != cudaSuccess) {
       free_solver(s);
       return set_err(PCFD_ERR_CUDA, "limiter init");
     }
@@ -3638,24 +3644,24 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
     for (int c = 0; c < ncol; c++) s->color_ptr[c + 1] += s->color_ptr[c];
     std::vector<int> rows(nn), fill(s->color_ptr.begin(), s->color_ptr.end() - 1);
     for (long long i = 0; i < nn; i++) rows[fill[color[i]]++] = (int)i;
-    TRY(dput(&s->d_ia, ia.data(), ia.size()));
-    TRY(dput(&s->d_ja, ja.data(), ja.size()));
-    TRY(dput(&s->d_pos_lr, pos_lr.data(), pos_lr.size()));
-    TRY(dput(&s->d_pos_rl, pos_rl.data(), pos_rl.size()));
-    TRY(dput(&s->d_color_rows, rows.data(), rows.size()));
-    TRY(dput(&s->d_cptr, s->color_ptr.data(), s->color_ptr.size()));
+    TRY(dput(s->stream, &s->d_ia, ia.data(), ia.size()));
+    TRY(dput(s->stream, &s->d_ja, ja.data(), ja.size()));
+    TRY(dput(s->stream, &s->d_pos_lr, pos_lr.data(), pos_lr.size()));
+    TRY(dput(s->stream, &s->d_pos_rl, pos_rl.data(), pos_rl.size()));
+    TRY(dput(s->stream, &s->d_color_rows, rows.data(), rows.size()));
+    TRY(dput(s->stream, &s->d_cptr, s->color_ptr.data(), s->color_ptr.size()));
     {
       std::vector<int4> desc(nn);
       for (long long g = 0; g < nn; g++) {
         const int i = rows[g];
         desc[g] = make_int4(i, ia[i] + 1, ia[i + 1] - ia[i] - 1, 0);
       }
-      TRY(dput(&s->d_rowdesc, desc.data(), desc.size()));
+      TRY(dput(s->stream, &s->d_rowdesc, desc.data(), desc.size()));
     }
     TRY(dalloc(&s->d_gbar, 2));
     TRY(dalloc(&s->d_sgs_err, 1));
-    CUDA_TRY(cudaMemset(s->d_gbar, 0, 2 * sizeof(unsigned int)));
-    CUDA_TRY(cudaMemset(s->d_sgs_err, 0, sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(s->d_gbar, 0, 2 * sizeof(unsigned int), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_sgs_err, 0, sizeof(int), s->stream));
     TRY(dalloc(&s->d_diag, (size_t)nn * 25));
     TRY(dalloc(&s->d_dlu, (size_t)nn * 25));
     TRY(dalloc(&s->d_dinv, (size_t)nn * 25 + 4));
@@ -3808,7 +3814,7 @@ PCFD_API int pcfd_forces(pcfd_solver_t h, const int* tags, int ntags, double* ou
   if (s->prm.viscous && (!s->have_grad || s->grad_arith != 0) && (rc = run_gradient(s, 0))) return rc;
   int* d_mask = nullptr;
   double* d_out = nullptr;
-  if ((rc = dput(&d_mask, mask.data(), mask.size()))) return rc;
+  if ((rc = dput(s->stream, &d_mask, mask.data(), mask.size()))) return rc;
   if ((rc = dalloc(&d_out, 6))) { cudaFree(d_mask); return rc; }
   const double Sconst = 110.4 / s->prm.ref_temperature;
   const double inv_retilde = s->prm.Re != 0.0 ? s->prm.mach / s->prm.Re : 0.0;

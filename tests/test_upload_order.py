@@ -1,7 +1,7 @@
 """Uploads are ordered before the kernels that read them.  A handle's stream is
 created non-blocking, so its kernels do not wait for the legacy stream, on which
 a copy from pageable memory may still be under way when cudaMemcpy returns: every
-upload is issued on the handle's own stream."""
+upload, and every clearing of device memory, is issued on the handle's own stream."""
 import re
 from pathlib import Path
 
@@ -14,12 +14,13 @@ from proteuscfd_gb300.chem import ChemModel
 CSRC = Path(__file__).resolve().parent.parent / "proteuscfd_gb300" / "csrc"
 
 
-@pytest.mark.parametrize("source", ["chem.cu"])
+@pytest.mark.parametrize("source", ["chem.cu", "solver.cu"])
 def test_no_upload_on_the_legacy_stream(source):
     text = (CSRC / source).read_text()
     assert "cudaStreamNonBlocking" in text
     uploads = [c for c in re.findall(r"cudaMemcpy\s*\([^;]*;", text) if "HostToDevice" in c]
     assert not uploads, uploads
+    assert not re.findall(r"cudaMemset\s*\([^;]*;", text)
 
 
 @pytest.mark.gpu
