@@ -22,14 +22,6 @@ template <>
 __device__ __forceinline__ __nv_bfloat16 to_store<__nv_bfloat16>(double v) { return __double2bfloat16(v); }
 
 __device__ __forceinline__ double ld_blk(const double* p) { return *p; }
-// an FP32 value as a double, exactly, on the integer pipes (the conversion
-// instruction runs on the FP64 pipe); zero, subnormal, infinite and NaN
-// values take the conversion
-__device__ __forceinline__ double widen(float f) {
-  const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
-  if (m - 0x00800000u >= 0x7f000000u) return m == 0u ? __hiloint2double((int)b, 0) : (double)f;
-  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + ((1023u - 127u) << 20))), (int)(b << 29));
-}
 __device__ __forceinline__ double ld_blk(const float* p) { return widen(*p); }
 __device__ __forceinline__ double ld_blk(const __nv_bfloat16* p) { return widen(__bfloat162float(*p)); }
 __device__ __forceinline__ float ld_blkf(const double* p) { return (float)*p; }

@@ -65,6 +65,15 @@ __device__ __forceinline__ float est_f32(double x) {
   return __uint_as_float(b | ((unsigned)hi & 0x80000000u));
 }
 
+// an FP32 value as a double, exactly, on the integer pipes (the conversion
+// instruction runs on the FP64 pipe); zero, subnormal, infinite and NaN
+// values take the conversion
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return m == 0u ? __hiloint2double((int)b, 0) : (double)f;
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + ((1023u - 127u) << 20))), (int)(b << 29));
+}
+
 // 1 / x: within 0.5 ulp + 2^-10 ulp
 __device__ __forceinline__ double recip(double x) {
   if (!seed_range(x)) return 1.0 / x;
@@ -73,13 +82,15 @@ __device__ __forceinline__ double recip(double x) {
   return fma(y0, fma(e, e, e), y0);
 }
 
-// a / b within 0.5 ulp + 2^-20 ulp: the quotient's residual formed exactly
+// a / b within 0.5 ulp + 2^-20 ulp: the quotient's residual formed exactly.
+// Its sign is such that a zero's quotient keeps its own (q - (b q - a) / b).
 __device__ __forceinline__ double quot(double a, double b) {
-  if (!seed_range(abs_bits(b)) || !(seed_range(abs_bits(a)) || abs_bits(a) == 0.0)) return a / b;
-  const double ra = recip(abs_bits(b));
-  const double r = __double2hiint(b) < 0 ? -ra : ra;
+  const double ab = abs_bits(b);
+  if (!seed_range(ab) || !(seed_range(abs_bits(a)) || abs_bits(a) == 0.0)) return a / b;
+  const double r = recip(ab);
   const double q = a * r;
-  return fma(fma(-b, q, a), r, q);
+  const double v = fma(-fma(ab, q, -a), r, q);
+  return __double2hiint(b) < 0 ? -v : v;
 }
 
 // Quotients by one denominator: its reciprocal is shared and each quotient
@@ -93,11 +104,11 @@ struct Quot64 {
   __device__ __forceinline__ double of(double a) const {
     if (!ok || !(abs_bits(a) == 0.0 || seed_range(abs_bits(a)))) return a / b;
     const double q = a * r;
-    return fma(fma(-b, q, a), r, q);
+    return fma(-fma(b, q, -a), r, q);
   }
 };
 
-// sqrt(x) and *inv = 1 / sqrt(x), each within 1 ulp
+// sqrt(x) and *inv = 1 / sqrt(x), each within 1 ulp (of the seeded range)
 __device__ __forceinline__ double sqrt_inv(double x, double* inv) {
   if (!seed_range(x)) {
     const double s = ::sqrt(x);
