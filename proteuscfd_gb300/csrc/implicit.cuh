@@ -35,11 +35,6 @@ __device__ __forceinline__ void numflux(const double* QL, const double* QR, cons
   if (kneecap5(f)) atomicAdd(&health[H_KNEECAP], 1ull);
 }
 
-// CompressibleEqnSet::ViscousJacobian (ucs/compressible.tcc:1633), laminar,
-// in the scalar type R (FP64; FP32 when the blocks are stored in FP32 or BF16).
-// QL/QR are the nodal 10-wide records (their stored pressure is used, as
-// GetPressure reads it); aL/aR are the left/right blocks with the sign the
-// reference scatters them with.
 // Quotients by one denominator: FP64 shares the reciprocal and corrects each
 // quotient by its residual (rounded as the operator rounds), FP32 divides.
 template <class R>
@@ -53,6 +48,11 @@ struct Den<double> : Quot64 {
   using Quot64::Quot64;
 };
 
+// CompressibleEqnSet::ViscousJacobian (ucs/compressible.tcc:1633), laminar,
+// in the scalar type R (FP64; FP32 when the blocks are stored in FP32 or BF16).
+// QL/QR are the nodal 10-wide records (their stored pressure is used, as
+// GetPressure reads it); aL/aR are the left/right blocks with the sign the
+// reference scatters them with.
 template <class R>
 __device__ void viscous_jacobian(const R* QL, const R* QR, const R* dx, R s2, R ax, R ay, R az, R aw, R gamma, R Pr,
                                  R inv_retilde, R S, R* aL, R* aR) {
@@ -1563,8 +1563,8 @@ __device__ __forceinline__ S max_eig(const S* QL, const S* QR, const V& a, S gam
 // The FP64 form: |theta| + c, the larger of |theta + c| and |theta - c|, from
 // the face sums (the halves cancel in the velocity and in c^2), reciprocal
 // and root from FP32 seeds: 28 FP64 instructions a face against 60 (the
-// kernel keeps the FP64 pipe 85 % busy; 64x48x48 box: 94 us a call before, 68
-// now)
+// kernel keeps the FP64 pipe 85 % busy; the time step's three launches on the
+// 64x48x48 box: 278 us before, 203 now)
 __device__ __forceinline__ double max_eig(const double* QL, const double* QR, const D4& a, double gamma) {
   const double s0 = QL[0] + QR[0], s1 = QL[1] + QR[1], s2 = QL[2] + QR[2], s3 = QL[3] + QR[3], s4 = QL[4] + QR[4];
   const double ir = recip(s0);

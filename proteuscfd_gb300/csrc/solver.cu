@@ -3257,7 +3257,7 @@ int lp_alloc(Solver* s) {
   const int n = s->nnode;
   lp->n = n;
   lp->nnz = 2LL * s->nedge;
-  lp->grid_red = std::min(nblk(n, 8), 4 * 152);
+  lp->grid_red = std::min(nblk(n, 8), 4 * s->nsm);
   lp->npb = std::max(LP_WG_CHUNK, nblk(n, 2 * s->nsm));  // two blocks a multiprocessor
   const int nwb = nblk(n, lp->npb);
   lp->grid_gather = std::min(nblk(n, 16), LP_GB_SM * s->nsm);
