@@ -457,8 +457,9 @@ __device__ void bc_inviscid_wall(S gamma, int no_cvbc, const S* QL, S pi, S* QR,
   }
 }
 
-// The generic forms for states the FP64 forms below leave (an average with a
-// density or pressure that is not positive), for the sub-iterations left
+// The generic forms for states the FP64 forms below leave (an average whose
+// density or pressure is not positive, or outside the seeds' range, where the
+// products of the two over- or underflow), for the sub-iterations left
 __device__ __noinline__ void bc_farfield_rest(double gamma, const double* Qinf, const double* QL, double pi,
                                               double* QR, double ax, double ay, double az, int nsub) {
   bc_farfield<double>(gamma, Qinf, QL, pi, QR, ax, ay, az, nsub);
@@ -498,7 +499,7 @@ __device__ __forceinline__ void bc_farfield64(double gamma, const double* Qinf, 
       theta = theta_ref<double>(0.5 * s0, 0.5 * s1, 0.5 * s2, 0.5 * s3, ax, ay, az);
     const double pavg = hgm1 * fma(-0.5, fma(s1, tu, fma(s2, tv, s3 * tw)), s4);
     const double gp = gamma * pavg, t0 = 0.5 * s0, a = gp * t0;
-    if (!(key_gt(t0, 0.0) && key_gt(gp, 0.0)) || not_finite(a) || not_finite(theta)) {
+    if (!(seed_range(t0) && seed_range(gp)) || not_finite(theta)) {
       bc_farfield_rest(gamma, Qinf, QL, pi, QR, ax, ay, az, kBcSubits - subit);
       return;
     }
@@ -553,7 +554,7 @@ __device__ __forceinline__ void bc_inviscid_wall64(double gamma, const double* Q
     const double s0 = rhoi + rb, is0 = recip(s0);
     const double pavg = hgm1 * fma(-0.5 * msq, is0, s4);
     const double t0 = 0.5 * s0, a = gamma * pavg * t0;
-    if (!(key_gt(t0, 0.0) && key_gt(pavg, 0.0)) || not_finite(a)) {
+    if (!(seed_range(t0) && seed_range(pavg))) {
       if (subit > 0) {
         QR[0] = rb; QR[1] = rb * ub; QR[2] = rb * vb; QR[3] = rb * wb;
         QR[4] = fma(pb, igm1, rb * hub2);
