@@ -1567,7 +1567,7 @@ __device__ __forceinline__ S max_eig(const S* QL, const S* QR, const V& a, S gam
 // 64x48x48 box: 278 us before, 203 now)
 __device__ __forceinline__ double max_eig(const double* QL, const double* QR, const D4& a, double gamma) {
   const double s0 = QL[0] + QR[0], s1 = QL[1] + QR[1], s2 = QL[2] + QR[2], s3 = QL[3] + QR[3], s4 = QL[4] + QR[4];
-  const double ir = recip(s0);
+  const double ir = recip_finite(s0);
   const double u = s1 * ir, v = s2 * ir, w = s3 * ir;
   const double c2 = (gamma * (gamma - 1.0)) * fma(-0.5, fma(s1, u, fma(s2, v, s3 * w)), s4) * ir;
   return abs_bits(fma(u, a.x, fma(v, a.y, w * a.z))) + root(c2);

@@ -82,6 +82,12 @@ __device__ __forceinline__ double recip(double x) {
   return fma(y0, fma(e, e, e), y0);
 }
 
+// 1 / x for a density whose product with 1 / x stands for 1 in what follows:
+// NaN instead of 0 for an infinite one
+__device__ __forceinline__ double recip_finite(double x) {
+  return seed_range(x) ? recip(x) : 1.0 / x + (x - x);
+}
+
 // a / b within 0.5 ulp + 2^-20 ulp: the quotient's residual formed exactly.
 // Its sign is such that a zero's quotient keeps its own (q - (b q - a) / b).
 __device__ __forceinline__ double quot(double a, double b) {

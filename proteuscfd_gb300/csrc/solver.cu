@@ -1655,7 +1655,7 @@ __device__ __forceinline__ void edge_visc64(const double* __restrict__ qL, const
                                             const double* __restrict__ h, const D4& a, const FluxK<double>& k, bool ho,
                                             double* fv) {
   const double s0 = qL[0] + qR[0], s1 = qL[1] + qR[1], s2 = qL[2] + qR[2], s3 = qL[3] + qR[3], s4 = qL[4] + qR[4];
-  const double is0 = recip(s0);
+  const double is0 = recip_finite(s0);
   const double u = s1 * is0, v = s2 * is0, w = s3 * is0;
   // T = gamma P / rho of the averaged state: the halves of P and rho cancel
   const double T = (k.gamma * k.gm1) * fma(-0.5, fma(s1, u, fma(s2, v, s3 * w)), s4) * is0;
