@@ -1053,13 +1053,13 @@ __device__ __forceinline__ void limit_node(int i, int k0, int k1, const int* __r
 // 1e-6 (2), and for 1 at any amplitude.
 // us a pass of the full evaluation over all neighbours / this one:
 //   53x37x29 box, noise of 1e-16, 1e-15, 1e-12, 1e-6, 1e-2 of the values
-//     1 Barth     126/121  222/130  193/130  193/110  192/93
-//     2 plain     201/128  334/151  274/142  273/120  274/98
-//     3 modified  137/72   137/72   137/73   138/79   137/75
+//     1 Barth     126/93   222/99   193/99   193/84   192/67
+//     2 plain     201/129  334/153  274/139  273/118  274/98
+//     3 modified  137/68   137/68   137/68   138/75   137/73
 //   128x96x96 box
-//     1           2198/1569  4130/1697  3438/1680  3440/1406  3443/1353
-//     2           3716/1613  6262/1861  4854/1765  4845/1489  4856/1430
-//     3           2546/1016  2546/1013  2546/1016  2546/1174  2546/1165
+//     1           2198/1429  4130/1527  3438/1530  3440/1228  3443/1166
+//     2           3716/1611  6262/1853  4854/1757  4845/1476  4856/1419
+//     3           2546/1016  2546/1019  2546/1021  2546/1176  2546/1171
 
 // dx of neighbour entry k, and grad.dx in the reference's rounding
 __device__ __forceinline__ double limit_gdx(int se, const double* __restrict__ eh, double g0, double g1, double g2) {
@@ -1088,12 +1088,27 @@ __device__ __forceinline__ double limit_value(double q, double qmin, double qmax
   return quot(r * r + 2.0 * r, r * r + r + 2.0);
 }
 
-// the smallest r over all neighbours, one equation
+// the smallest r over all neighbours, one equation; the modified form's running
+// minimum as a fraction compared by cross-multiplication, as limit_node keeps it
 template <int LIM>
 __device__ __noinline__ double limit_exact(int k0, int k1, const int* __restrict__ nedg,
                                            const double* __restrict__ eh, double q, double qmin, double qmax,
                                            double g0, double g1, double g2, double ep2) {
   double v = 1.0;
+  if (LIM == 3) {
+    const double dpp = qmax - q, dpm = qmin - q;
+    double d = 1.0;
+    for (int k = k0; k < k1; k++) {
+      const double Q = __dadd_rn(q, limit_gdx(nedg[k], eh, g0, g1, g2));
+      const double DM = Q - q, DP = Q > q ? dpp : dpm, C1 = fma(DP, DP, ep2);
+      const double num = fma(DM, DP + DP, C1), den = fma(DM, fma(2.0, DM, DP), C1);
+      if (num * d < v * den) {
+        v = num;
+        d = den;
+      }
+    }
+    return d == 1.0 ? v : quot(v, d);
+  }
   for (int k = k0; k < k1; k++) {
     const double r = limit_value<LIM>(q, qmin, qmax, limit_gdx(nedg[k], eh, g0, g1, g2), ep2);
     if (r < v) v = r;
@@ -1120,6 +1135,7 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
   bool flat[NEQN];   // Venkatakrishnan: some neighbour's extrapolation leaves the value as it is (r = 3/4)
   bool nil[NEQN];    // Barth: some neighbour's r is certainly 0
   bool range[NEQN];  // operands FP32 can square
+  bool wild[NEQN];   // some neighbour's r has no estimate: too small, too large, not finite
 #pragma unroll
   for (int t = 0; t < NEQN; t++) {
     const double DPP = key_value(kmx[t]) - qi[t], DPM = key_value(kmn[t]) - qi[t];
@@ -1129,7 +1145,7 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
     u1[t] = u2[t] = v3[t] = -inf;
     m1[t] = m2[t] = 0.0f;
     e1[t] = e2[t] = k0;
-    flat[t] = nil[t] = false;
+    flat[t] = nil[t] = wild[t] = false;
     range[t] = ep2f > 1.0e-30f && ep2f < 1.0e30f && qe[t] < 1.0e15f && fabsf(dpp[t]) < 1.0e15f &&
                fabsf(dpm[t]) < 1.0e15f &&
                (LIM == 3 || ((dpp[t] != 0.0f || DPP == 0.0) && (dpm[t] != 0.0f || DPM == 0.0)));
@@ -1162,6 +1178,7 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
       const float dp = dm > 0.0f ? dpp[t] : dpm[t];
       const float am = fabsf(dm), ap = fabsf(dp);
       float u, m;
+      bool fits;
       if (LIM == 3) {
         // u = DM (2 DM - DP) / den.  Each operand is within 2^-22, den keeps
         // at least 0.47 of its terms' magnitudes, so u is within 2.9e-6 a /
@@ -1170,10 +1187,7 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
         const float rd = rcp_f32(dp * dp + ep2f + dm * (dp + 2.0f * dm));
         u = dm * (2.0f * dm - dp) * rd;
         m = (3.0e-6f * am * a + 4.0e-16f * qe[t] * (a + 2.0f * am)) * rd;
-        if (!(range[t] && am < 1.0e15f)) {
-          u = 0.0f;
-          m = inf;
-        }
+        fits = range[t] && am < 1.0e15f;
       } else {
         // r is a function of DP / DM with a slope of at most 1, flat where the
         // ratio is large, and the ratio is within 2^-20 of itself (3e-6 covers
@@ -1181,14 +1195,12 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
         const float tr = dp * rcp_f32(dm);
         u = LIM == 1 ? 1.0f - fminf(fmaxf(tr, 0.0f), 1.0f) : (2.0f - tr) * rcp_f32(tr * tr + tr + 2.0f);
         m = 3.0e-6f;
-        if (!(range[t] && am > 1.0e-30f && am < 1.0e15f && fabsf(tr) < 1.0e15f)) {
-          u = 0.0f;
-          m = inf;
-        } else if (dp == 0.0f) {  // r is 0
+        fits = range[t] && am > 1.0e-30f && am < 1.0e15f && fabsf(tr) < 1.0e15f;
+        if (fits && dp == 0.0f) {  // r is 0
           if (LIM == 1) nil[t] = true;
           u = 1.0f;
           m = 0.0f;
-        } else if (LIM == 1 && tr < -1.0e-5f) {
+        } else if (LIM == 1 && fits && tr < -1.0e-5f) {
           nil[t] = true;
         }
       }
@@ -1197,7 +1209,8 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
       const bool free = dm * dp > 0.0f &&
                         ap > (LIM == 1 ? 1.00001f : 2.00001f) * am + (LIM == 3 ? 4.0e-16f * qe[t] : 0.0f);
       if (still) flat[t] = true;
-      if (still || free || twin) {
+      if (still || free || twin || !fits) {
+        if (!(still || free || twin)) wild[t] = true;
         u = -inf;
         m = 0.0f;
       }
@@ -1227,9 +1240,9 @@ __device__ __forceinline__ void limit_node64(int i, int k0, int k1, const int* _
     const float low = u1[t] - m1[t], second = u2[t] + m2[t];
     if (LIM == 1 && nil[t]) {
       v = 0.0;
-    } else if (fmaxf(fmaxf(u1[t] + m1[t], second), v3[t]) < 5.0e-17f) {
+    } else if (!wild[t] && fmaxf(fmaxf(u1[t] + m1[t], second), v3[t]) < 5.0e-17f) {
       v = 1.0;  // no neighbour below 1 - 2^-54
-    } else if (v3[t] > fmaxf(low, 0.0f)) {
+    } else if (wild[t] || v3[t] > fmaxf(low, 0.0f)) {
       v = limit_exact<LIM>(k0, k1, nedg, eh, qi[t], key_value(kmn[t]), key_value(kmx[t]), gi[3 * t], gi[3 * t + 1],
                            gi[3 * t + 2], ep2);
     } else {
