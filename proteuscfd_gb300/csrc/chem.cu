@@ -1238,7 +1238,13 @@ __global__ void __launch_bounds__(128) k_chem_limiter(long long nnode, const pcf
       const bool up = key_gt(Q, qi[j]);
       const double DP = up ? dpp[j] : dpm[j], C1 = up ? cp[j] : cm[j];
       const double num = fma(DM, DP + DP, C1), den = fma(DM, fma(2.0, DM, DP), C1);
-      if (key_gt(bn[j] * den, num * bd[j])) {
+      if (!seed_range(den)) {  // not finite, or a product may over- or underflow: by the quotients
+        const double t = num / den;
+        if (t < (bd[j] == 1.0 ? bn[j] : bn[j] / bd[j])) {
+          bn[j] = t;
+          bd[j] = 1.0;
+        }
+      } else if (key_gt(bn[j] * den, num * bd[j])) {
         bn[j] = num;
         bd[j] = den;
       }
