@@ -260,9 +260,10 @@ __device__ __forceinline__ void rates_with(const pcfd_chem_model& m, const ChemD
 }
 
 // rho / MW from the stored reciprocal, corrected by the quotient's residual
+// (infinite and overflowing ones as they are)
 __device__ __forceinline__ double molar(const pcfd_chem_model& m, const ChemDerived& d, int k, double rho) {
   const double q = rho * d.imw[k];
-  return fma(fma(-m.mw[k], q, rho), d.imw[k], q);
+  return not_finite(q) ? q : fma(-fma(m.mw[k], q, -rho), d.imw[k], q);
 }
 
 // mass production rates of one node (rhoi [ns] kg/m^3, T K -> wdot [ns]).

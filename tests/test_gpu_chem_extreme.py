@@ -3,8 +3,8 @@ give."""
 import numpy as np
 import pytest
 
-from chem_cases import fr_records, fr_states, mechanism
-from oracle_lib import OracleChemState
+from chem_cases import fr_records, fr_states, mechanism, states
+from oracle_lib import OracleChemState, chem_rates
 from proteuscfd_gb300 import Mesh
 from proteuscfd_gb300.chem import ChemModel, model_struct
 
@@ -33,4 +33,17 @@ def test_limiter_beside_infinite_values(chi, value):
         with np.errstate(invalid="ignore"):
             assert np.array_equal(np.isnan(lim[others]), np.isnan(lo[others])), component
             assert np.nanmax(np.abs(lim - lo)[others]) <= 1e-12
+    C.close()
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+@pytest.mark.parametrize("species", range(5))
+def test_rates_of_infinite_densities(species, value):
+    """Infinite rates are infinite and NaN ones NaN where the oracle's are."""
+    rho, T = states(300, seed=7)
+    rho[::7, species] = value
+    C = ChemModel(mechanism())
+    w, wo = C.production_rates(rho, T), chem_rates(model_struct(mechanism()), rho, T)
+    assert np.array_equal(np.isnan(w), np.isnan(wo))
+    assert np.array_equal(w[np.isinf(wo)], wo[np.isinf(wo)]) and np.array_equal(np.isinf(w), np.isinf(wo))
     C.close()
