@@ -21,9 +21,9 @@ namespace pcfd {
 
 // positive with a binary exponent of -100 .. 99: one unsigned compare on the
 // high word
-__device__ __forceinline__ bool seed_range(double x) {
-  return (unsigned)(__double2hiint(x) - ((1023 - 100) << 20)) < (200u << 20);
-}
+constexpr unsigned kSeedSpan = 200u << 20;
+__device__ __forceinline__ unsigned seed_offset(double x) { return (unsigned)(__double2hiint(x) - ((1023 - 100) << 20)); }
+__device__ __forceinline__ bool seed_range(double x) { return seed_offset(x) < kSeedSpan; }
 // |v| without the sign bit
 __device__ __forceinline__ double abs_bits(double v) {
   return __hiloint2double(__double2hiint(v) & 0x7fffffff, __double2loint(v));

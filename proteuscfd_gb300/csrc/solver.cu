@@ -1939,13 +1939,17 @@ int dalloc(T** p, size_t n) {
 
 // a new device array with h's values, on the handle's stream st: it does not
 // wait for the legacy stream, on which a copy from pageable memory may still
-// be under way when cudaMemcpy returns
+// be under way when cudaMemcpy returns.  The caller keeps h until it has
+// synchronised the stream.
 template <class T>
 int dput(cudaStream_t st, T** p, const T* h, size_t n) {
   int rc = dalloc(p, n);
   if (rc || n == 0) return rc;
   CUDA_TRY(cudaMemcpyAsync(*p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(cudaStreamSynchronize(st));
+  return PCFD_OK;
+}
+int sync_puts(Solver* s) {
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
   return PCFD_OK;
 }
 
@@ -1953,6 +1957,7 @@ void free_learned(Learned* lp);
 
 void free_solver(Solver* s) {
   if (!s) return;
+  if (s->stream) cudaStreamSynchronize(s->stream);
   free_learned(s->lp);
   void* ptrs[] = {s->d_en, s->d_ea, s->d_eh, s->d_bn, s->d_ba, s->d_bbc, s->d_btw, s->d_bfactag, s->d_bnrm, s->d_xyz,
                   s->d_vol, s->d_nptr, s->d_nedg, s->d_nnbr, s->d_lsq, s->d_bptr, s->d_bhe, s->d_bgnode,
@@ -3547,6 +3552,7 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
     s->nbgslot = (int)slot.size();
     TRY(dput(s->stream, &s->d_bgslot, slot.data(), slot.size()));
     TRY(dalloc(&s->d_bgqr, std::max<size_t>(slot.size(), 1) * NVARS));
+    TRY(sync_puts(s));
   }
   TRY(dput(s->stream, &s->d_bind, bind.data(), bind.size()));
   TRY(dalloc(&s->d_clipflag, (size_t)nn));
@@ -3671,6 +3677,7 @@ PCFD_API int pcfd_create(const pcfd_mesh_view* m, const pcfd_params* prm, pcfd_s
         desc[g] = make_int4(i, ia[i] + 1, ia[i + 1] - ia[i] - 1, 0);
       }
       TRY(dput(s->stream, &s->d_rowdesc, desc.data(), desc.size()));
+      TRY(sync_puts(s));
     }
     TRY(dalloc(&s->d_gbar, 2));
     TRY(dalloc(&s->d_sgs_err, 1));
